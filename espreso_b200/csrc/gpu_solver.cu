@@ -200,6 +200,25 @@ void launch_pdl(void (*kernel)(KA...), dim3 grid, dim3 block, size_t smem, cudaS
     CUDA_CHECK(cudaLaunchKernelEx(&cfg, kernel, static_cast<KA>(args)...));
 }
 
+// the same for thread-block clusters of `cluster` CTAs (the grid is a multiple of it)
+template <typename... KA, typename... A>
+void launch_cluster(void (*kernel)(KA...), int cluster, dim3 grid, dim3 block, size_t smem, cudaStream_t stream, A... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cudaLaunchAttribute at[2];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = (unsigned)cluster;
+    at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+    at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[1].val.programmaticStreamSerializationAllowed = pdl_enabled() ? 1 : 0;
+    cfg.attrs = at;
+    cfg.numAttrs = 2;
+    CUDA_CHECK(cudaLaunchKernelEx(&cfg, kernel, static_cast<KA>(args)...));
+}
+
 template <typename T>
 __device__ __forceinline__ T warp_sum(T v) {
 #pragma unroll
@@ -1191,6 +1210,12 @@ struct KplusDev {
     const int *cptr;
     const int *rows;
     const long long *tpre;   // 32-blocks of the subdomains before d (vectors of kplus_mma_kernel in global memory)
+    // the same tiles as symmetric bit rows: bit Y of row X (mw[d] words from mask[moff[d]] on) is set when
+    // tile (max(X, Y), min(X, Y)) is not all zero
+    const int *mw;
+    const long long *moff;
+    const unsigned *mask;
+    const int *order;        // subdomains by descending number of nonzero tiles
 };
 
 // nz[t] = 1 when tile t holds a nonzero (one warp per tile)
@@ -1219,94 +1244,198 @@ __device__ __forceinline__ long long ltile(int T, int I, int J) {
     return (long long)J * T - (long long)J * (J - 1) / 2 + (I - J);
 }
 
-__global__ void __launch_bounds__(256) kplus_kernel(KplusDev K, const double *in, double *out, int mode) {
-    extern __shared__ double v[];
-    __shared__ double part[8][32];
-    const int d = blockIdx.x;
+// Triangular sweep of one subdomain by a cluster of C CTAs (KP_WARPS warps each).
+//
+// One CTA per subdomain reads its factor at what one SM can request, and a barrier pair per 32-column
+// step leaves the diagonal step alone on the critical path, so the sweep was bound by latency whenever
+// the subdomains did not fill the chip several times over.  Here step s publishes its 32 solved values
+// to every CTA of the cluster, and the target blocks t > s are dealt to the warps of the whole cluster
+// (warp t mod NW), each block to one warp for the whole sweep: its partial sums need no atomics and no
+// barrier.  The warp that owns block s + 1 applies its tile first, solves the diagonal block (staged by
+// cp.async since its previous turn) and publishes it while the others still work on step s; every other
+// warp has arrived at the cluster barrier of step s + 1 before its own tiles, so the barrier costs the
+// publishing warp's path only.  Every CTA keeps the whole vector in shared memory.
+// Per pass, one CTA per subdomain before / clusters now: 64 subdomains of 8^3 elasticity elements (0.64 GB
+// of nonzero tiles) 905 / 255 us, 64 uneven ones of up to 7,560 DOFs (largest 0.14 GB) 5.2 / 1.5 ms, 27
+// of 6^3 271 / 100 us; 512 of 10^3 heat elements fill the chip either way (592 us, clusters of one).
+constexpr int KP_WARPS = 8;
+
+__device__ __forceinline__ unsigned cluster_size_x() {
+    unsigned v;
+    asm volatile("mov.u32 %0, %%cluster_nctaid.x;" : "=r"(v));
+    return v;
+}
+__device__ __forceinline__ unsigned cluster_rank_x() {
+    unsigned v;
+    asm volatile("mov.u32 %0, %%cluster_ctaid.x;" : "=r"(v));
+    return v;
+}
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire;" ::: "memory"); }
+// the same shared-memory variable in CTA `rank` of the cluster
+__device__ __forceinline__ void st_cluster(double *p, unsigned rank, double v) {
+    unsigned a;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"((unsigned)__cvta_generic_to_shared(p)), "r"(rank));
+    asm volatile("st.shared::cluster.f64 [%0], %1;" ::"r"(a), "d"(v) : "memory");
+}
+
+struct KpTile {
+    uint4 u[16];
+};
+__device__ __forceinline__ void kp_load(KpTile &t, const uint4 *tp, int lane) {
+#pragma unroll
+    for (int q = 0; q < 16; ++q) t.u[q] = ld_stream(tp + q * 32 + lane);
+}
+// entry idx of tile * x (FWD) or tile^T * x: one entry per lane, idx = 2 (lane % 16) + lane / 16; chunk(q)
+// is the lane's 16-byte chunk q * 32 + lane of the tile
+template <bool FWD, typename F>
+__device__ __forceinline__ double kp_apply(F chunk, const double *x, int lane) {
+    const int cq = lane % 16, h = lane / 16;
+    if (FWD) {
+        const double x0 = x[2 * cq], x1 = x[2 * cq + 1];
+        double rs[16];
+#pragma unroll
+        for (int q = 0; q < 16; ++q) {
+            const uint4 u = chunk(q);
+            rs[q] = __hiloint2double(u.y, u.x) * x0 + __hiloint2double(u.w, u.z) * x1;
+        }
+        return reduce_scatter<16, 0>(rs, lane);
+    }
+    double cs[2] = {0.0, 0.0};
+#pragma unroll
+    for (int q = 0; q < 16; ++q) {
+        const uint4 u = chunk(q);
+        const double xr = x[2 * q + h];
+        cs[0] += __hiloint2double(u.y, u.x) * xr;
+        cs[1] += __hiloint2double(u.w, u.z) * xr;
+    }
+    return reduce_scatter<2, 4>(cs, lane);
+}
+
+// FWD: v[32 lo ..) := L^-1 v over the blocks lo .. T-1; else v := L^-T v, blocks T-1 down to lo.  v is
+// whole and the same in every CTA on entry (after a cluster barrier) and on return.
+// dbuf: 8 KB per warp, or null (the diagonal tiles are then read when they are needed).
+template <bool FWD>
+__device__ void kp_sweep(const uint4 *tiles, const unsigned *mask, int mw, int T, int lo, double *v, uint4 *dbuf) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int C = (int)cluster_size_x(), NW = KP_WARPS * C, W = warp * C + (int)cluster_rank_x();
+    const int steps = T - lo, idx = 2 * (lane % 16) + lane / 16;
+    auto blk = [&](int s) { return FWD ? lo + s : T - 1 - s; };
+    auto tile = [&](int s, int t) {   // tile coupling steps s <= t
+        const int a = blk(s), b = blk(t);
+        return tiles + (size_t)(FWD ? ltile(T, b, a) : ltile(T, a, b)) * (TILE * 16);
+    };
+    uint4 *mydiag = dbuf ? dbuf + warp * (TILE * 16) : nullptr;
+    auto stage_diag = [&](int s) {
+        if (!mydiag || s >= steps) return;
+        const uint4 *src = tile(s, s);
+#pragma unroll
+        for (int q = 0; q < 16; ++q)
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((unsigned)__cvta_generic_to_shared(mydiag + q * 32 + lane)),
+                         "l"(src + q * 32 + lane)
+                         : "memory");
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    // solve the diagonal block of step s from this CTA's finished v and publish it (one warp)
+    auto publish = [&](int s) {
+        const uint4 *dp = mydiag ? mydiag : tile(s, s);
+        asm volatile("cp.async.wait_group 0;" ::: "memory");   // each lane reads what it copied itself
+        double *vb = v + TILE * blk(s);
+        __syncwarp();
+        const double y = kp_apply<FWD>([&](int q) { return dp[q * 32 + lane]; }, vb, lane);
+        __syncwarp();
+        for (int r = 0; r < C; ++r) st_cluster(vb + idx, (unsigned)r, y);
+        __syncwarp();
+        stage_diag(s + NW);
+    };
+    if (steps <= 0) return;   // the same for the whole cluster
+    stage_diag(W);
+    if (W == 0) publish(0);
+    cluster_arrive();
+    for (int s = 0; s < steps; ++s) {
+        const unsigned *mrow = mask + (size_t)blk(s) * mw;
+        auto present = [&](int t) { const int b = blk(t); return (mrow[b >> 5] >> (b & 31)) & 1u; };
+        int t = s + 1 + (W - (s + 1) % NW + NW) % NW;
+        const bool crit = t == s + 1 && t < steps;
+        auto next = [&] { while (t < steps && !present(t)) t += NW; };
+        next();
+        KpTile a;
+        if (t < steps && (!crit || t == s + 1)) kp_load(a, tile(s, t), lane);
+        cluster_wait();                                   // block s is solved in every CTA
+        const double *x = v + TILE * blk(s);
+        if (crit) {
+            if (t == s + 1) {
+                v[TILE * blk(t) + idx] -= kp_apply<FWD>([&](int q) { return a.u[q]; }, x, lane);
+                t += NW;
+                next();
+            }
+            publish(s + 1);
+            cluster_arrive();
+            if (t < steps) kp_load(a, tile(s, t), lane);
+        } else if (s + 1 < steps) {
+            cluster_arrive();
+        }
+        while (t < steps) {
+            const double y = kp_apply<FWD>([&](int q) { return a.u[q]; }, x, lane);
+            double *vt = v + TILE * blk(t) + idx;
+            t += NW;
+            next();
+            if (t < steps) kp_load(a, tile(s, t), lane);
+            *vt -= y;
+        }
+    }
+    asm volatile("cp.async.wait_all;" ::: "memory");
+}
+
+// Shared memory of the sweeps: the vector (vblocks blocks), then, as far as they fit, the staged diagonal
+// tiles (KPS_DIAG) and a copy of the subdomain's bit rows (KPS_MASK).
+enum { KPS_DIAG = 1, KPS_MASK = 2 };
+struct KpSmem {
+    int vblocks, parts;
+};
+__device__ __forceinline__ uint4 *kp_dbuf(double *v, KpSmem sm) {
+    return sm.parts & KPS_DIAG ? reinterpret_cast<uint4 *>(v + (size_t)TILE * sm.vblocks) : nullptr;
+}
+__device__ const unsigned *kp_mask(const KplusDev &K, int d, double *v, KpSmem sm) {
+    const unsigned *g = K.mask + K.moff[d];
+    if (!(sm.parts & KPS_MASK)) return g;
+    unsigned *m = reinterpret_cast<unsigned *>(v + (size_t)TILE * sm.vblocks + (sm.parts & KPS_DIAG ? KP_WARPS * TILE * TILE : 0));
+    for (int i = threadIdx.x; i < K.tn[d] * K.mw[d]; i += blockDim.x) m[i] = __ldg(g + i);
+    return m;
+}
+
+__global__ void __launch_bounds__(KP_WARPS * 32, 2) kplus_kernel(KplusDev K, const double *in, double *out, int mode,
+                                                                 KpSmem sm) {
+    pdl_enter();
+    extern __shared__ __align__(16) double v[];
+    const int C = (int)cluster_size_x(), rank = (int)cluster_rank_x();
+    const int d = K.order[blockIdx.x / C];
     const int n = K.n[d], T = K.tn[d], o = K.doff[d];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
     const int *pos = K.pos + o;
     const uint4 *tiles = reinterpret_cast<const uint4 *>(K.L) + (size_t)K.tile0[d] * (TILE * 16);
-    const double *dtiles = K.L + (size_t)K.tile0[d] * TILE * TILE;
-    const int *cp = K.cptr + K.cbase[d];
+    const unsigned *mask = kp_mask(K, d, v, sm);
+    uint4 *dbuf = kp_dbuf(v, sm);
     for (int i = threadIdx.x; i < TILE * T; i += blockDim.x) v[i] = 0.0;
     __syncthreads();
     for (int i = threadIdx.x; i < n; i += blockDim.x) v[pos[i]] = in[o + i];
-    __syncthreads();
-    const int cq = lane % 16, h = lane / 16, idx = 2 * cq + h;
+    cluster_arrive();
+    cluster_wait();
     const int jt = mode == KPLUS_FULL ? 0 : K.jt[d];
     double *zs = K.z + o;
     // forward: L y = f (rows before block jt are zero in mode 2, so their steps are skipped)
-    for (int J = (mode == KPLUS_PRIMAL ? jt : 0); J < T; ++J) {
-        if (warp == 0) {
-            // y_J = inv(L_JJ) v_J: lane r forms row r (zero above the diagonal)
-            const double *row = dtiles + (size_t)ltile(T, J, J) * TILE * TILE + lane * TILE;
-            const double vr = v[TILE * J + lane];
-            double s0 = 0.0, s1 = 0.0;
-#pragma unroll
-            for (int k = 0; k < TILE; k += 2) {
-                s0 += row[k] * __shfl_sync(FULL, vr, k);
-                s1 += row[k + 1] * __shfl_sync(FULL, vr, k + 1);
-            }
-            v[TILE * J + lane] = s0 + s1;
-        }
-        __syncthreads();
-        for (int q = cp[J] + 1 + warp; q < cp[J + 1]; q += nw) {
-            const int I = K.rows[q];
-            const uint4 *tp = tiles + (size_t)ltile(T, I, J) * (TILE * 16);
-            double rs[16];
-            const double x0 = v[TILE * J + 2 * cq], x1 = v[TILE * J + 2 * cq + 1];
-#pragma unroll
-            for (int q = 0; q < 16; ++q) {
-                uint4 u = ld_stream(tp + q * 32 + lane);
-                rs[q] = __hiloint2double(u.y, u.x) * x0 + __hiloint2double(u.w, u.z) * x1;
-            }
-            double r = reduce_scatter<16, 0>(rs, lane);
-            v[TILE * I + idx] -= r;
-        }
-        __syncthreads();
-    }
+    kp_sweep<true>(tiles, mask, K.mw[d], T, mode == KPLUS_PRIMAL ? jt : 0, v, dbuf);
+    __syncthreads();
     if (mode == KPLUS_TOUCHED) {
-        for (int i = threadIdx.x; i < n; i += blockDim.x) zs[i] = v[i];
-        __syncthreads();
+        for (int i = rank * blockDim.x + threadIdx.x; i < n; i += C * blockDim.x) zs[i] = v[i];
     } else if (mode == KPLUS_PRIMAL) {
         for (int i = threadIdx.x; i < n; i += blockDim.x) v[i] += zs[i];
-        __syncthreads();
     }
+    cluster_arrive();
+    cluster_wait();
     // backward: L^T x = y (in mode 1 only down to block jt)
-    for (int J = T - 1; J >= (mode == KPLUS_TOUCHED ? jt : 0); --J) {
-        double cpart = 0.0;
-        for (int q = cp[J] + 1 + warp; q < cp[J + 1]; q += nw) {
-            const int I = K.rows[q];
-            const uint4 *tp = tiles + (size_t)ltile(T, I, J) * (TILE * 16);
-            double cs[2] = {0.0, 0.0};
-#pragma unroll
-            for (int q = 0; q < 16; ++q) {
-                uint4 u = ld_stream(tp + q * 32 + lane);
-                double xr = v[TILE * I + 2 * q + h];
-                cs[0] += __hiloint2double(u.y, u.x) * xr;
-                cs[1] += __hiloint2double(u.w, u.z) * xr;
-            }
-            cpart += reduce_scatter<2, 4>(cs, lane);
-        }
-        part[warp][idx] = cpart;
-        __syncthreads();
-        if (warp == 0) {
-            double vc = v[TILE * J + lane];
-            for (int w = 0; w < nw; ++w) vc -= part[w][lane];
-            // x_J = inv(L_JJ)^T v_J: lane c forms column c of inv(L_JJ)
-            const double *tile = dtiles + (size_t)ltile(T, J, J) * TILE * TILE;
-            double s0 = 0.0, s1 = 0.0;
-#pragma unroll
-            for (int k = 0; k < TILE; k += 2) {
-                s0 += tile[k * TILE + lane] * __shfl_sync(FULL, vc, k);
-                s1 += tile[(k + 1) * TILE + lane] * __shfl_sync(FULL, vc, k + 1);
-            }
-            v[TILE * J + lane] = s0 + s1;
-        }
-        __syncthreads();
-    }
-    for (int i = threadIdx.x; i < n; i += blockDim.x) out[o + i] = v[pos[i]];
+    kp_sweep<false>(tiles, mask, K.mw[d], T, mode == KPLUS_TOUCHED ? jt : 0, v, dbuf);
+    __syncthreads();
+    for (int i = rank * blockDim.x + threadIdx.x; i < n; i += C * blockDim.x) out[o + i] = v[pos[i]];
 }
 
 // Implicit F apply (the reference's default without explicit Schur complements,
@@ -1315,16 +1444,16 @@ __global__ void __launch_bounds__(256) kplus_kernel(KplusDev K, const double *in
 // B_i^T x is zero at the untouched DOFs, which the factor order puts first, and only the touched
 // DOFs are read back, so the forward pass starts and the backward pass stops at the first touched
 // 32-block: both passes read only the factor's trailing touched part L_TT (its tiles that are not
-// all zero).  One CTA per subdomain writes the unassembled local product, as the tile SYMV does.
+// all zero).  The cluster of a subdomain writes the unassembled local product, as the tile SYMV does.
 // MODE 0: x = src, out += S x.  MODE 1 (PCG loop): x = src + beta src2 (direction p = y + beta p),
 // out = S x and p.Ap into SC_PAP.
 template <int MODE>
-__global__ void __launch_bounds__(256) kplus_dual_kernel(KplusDev K, DevProblem P, const int *rdof,
-                                                         const double *rsign, const double *src, const double *src2,
-                                                         double *out, int slot) {
+__global__ void __launch_bounds__(KP_WARPS * 32, 2) kplus_dual_kernel(KplusDev K, DevProblem P, const int *rdof,
+                                                                      const double *rsign, const double *src,
+                                                                      const double *src2, double *out, int slot,
+                                                                      KpSmem sm) {
     pdl_enter();
-    extern __shared__ double v[];
-    __shared__ double part[8][32];
+    extern __shared__ __align__(16) double v[];
     __shared__ double sh[32];
     double beta = 0.0;
     if (MODE == 1) {
@@ -1332,84 +1461,32 @@ __global__ void __launch_bounds__(256) kplus_dual_kernel(KplusDev K, DevProblem 
         if (skip_iter(P.st, iter)) return;
         beta = (iter == 0) ? 0.0 : P.scal[SC_RHO] / P.rho_hist[iter - 1];
     }
-    const int d = blockIdx.x;
+    const int C = (int)cluster_size_x(), rank = (int)cluster_rank_x();
+    const int d = K.order[blockIdx.x / C];
     const int T = K.tn[d], o = K.doff[d];
     const int e0 = P.loff[d], e1 = P.loff[d + 1];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
     const int *pos = K.pos + o;
     const uint4 *tiles = reinterpret_cast<const uint4 *>(K.L) + (size_t)K.tile0[d] * (TILE * 16);
-    const double *dtiles = K.L + (size_t)K.tile0[d] * TILE * TILE;
-    const int *cp = K.cptr + K.cbase[d];
+    const unsigned *mask = kp_mask(K, d, v, sm);
+    uint4 *dbuf = kp_dbuf(v, sm);
     const int jt = K.jt[d];
     for (int i = TILE * jt + threadIdx.x; i < TILE * T; i += blockDim.x) v[i] = 0.0;
     __syncthreads();
-    // B^T x: several multipliers (Dirichlet and gluing rows) may share a DOF
+    // B^T x: several multipliers (Dirichlet and gluing rows) may share a DOF.  A warp's own block is
+    // summed by its own CTA only, so the copies need not agree to the last bit.
     for (int e = e0 + threadIdx.x; e < e1; e += blockDim.x) {
         const double xv = (MODE == 1) ? src[e] + beta * src2[e] : src[e];
         atomicAdd(&v[pos[rdof[e] - o]], rsign[e] * xv);
     }
+    cluster_arrive();
+    cluster_wait();
+    kp_sweep<true>(tiles, mask, K.mw[d], T, jt, v, dbuf);    // L y = B^T x
+    cluster_arrive();
+    cluster_wait();
+    kp_sweep<false>(tiles, mask, K.mw[d], T, jt, v, dbuf);   // L^T z = y, down to the first touched block
     __syncthreads();
-    const int cq = lane % 16, h = lane / 16, idx = 2 * cq + h;
-    for (int J = jt; J < T; ++J) {   // forward: L y = B^T x
-        if (warp == 0) {
-            const double *row = dtiles + (size_t)ltile(T, J, J) * TILE * TILE + lane * TILE;
-            const double vr = v[TILE * J + lane];
-            double s0 = 0.0, s1 = 0.0;
-#pragma unroll
-            for (int k = 0; k < TILE; k += 2) {
-                s0 += row[k] * __shfl_sync(FULL, vr, k);
-                s1 += row[k + 1] * __shfl_sync(FULL, vr, k + 1);
-            }
-            v[TILE * J + lane] = s0 + s1;
-        }
-        __syncthreads();
-        for (int q = cp[J] + 1 + warp; q < cp[J + 1]; q += nw) {
-            const int I = K.rows[q];
-            const uint4 *tp = tiles + (size_t)ltile(T, I, J) * (TILE * 16);
-            double rs[16];
-            const double x0 = v[TILE * J + 2 * cq], x1 = v[TILE * J + 2 * cq + 1];
-#pragma unroll
-            for (int k = 0; k < 16; ++k) {
-                const uint4 u = ld_stream(tp + k * 32 + lane);
-                rs[k] = __hiloint2double(u.y, u.x) * x0 + __hiloint2double(u.w, u.z) * x1;
-            }
-            v[TILE * I + idx] -= reduce_scatter<16, 0>(rs, lane);
-        }
-        __syncthreads();
-    }
-    for (int J = T - 1; J >= jt; --J) {   // backward: L^T z = y, down to the first touched block
-        double cpart = 0.0;
-        for (int q = cp[J] + 1 + warp; q < cp[J + 1]; q += nw) {
-            const int I = K.rows[q];
-            const uint4 *tp = tiles + (size_t)ltile(T, I, J) * (TILE * 16);
-            double cs[2] = {0.0, 0.0};
-#pragma unroll
-            for (int k = 0; k < 16; ++k) {
-                const uint4 u = ld_stream(tp + k * 32 + lane);
-                const double xr = v[TILE * I + 2 * k + h];
-                cs[0] += __hiloint2double(u.y, u.x) * xr;
-                cs[1] += __hiloint2double(u.w, u.z) * xr;
-            }
-            cpart += reduce_scatter<2, 4>(cs, lane);
-        }
-        part[warp][idx] = cpart;
-        __syncthreads();
-        if (warp == 0) {
-            double vc = v[TILE * J + lane];
-            for (int w = 0; w < nw; ++w) vc -= part[w][lane];
-            const double *tile = dtiles + (size_t)ltile(T, J, J) * TILE * TILE;
-            double s0 = 0.0, s1 = 0.0;
-#pragma unroll
-            for (int k = 0; k < TILE; k += 2) {
-                s0 += tile[k * TILE + lane] * __shfl_sync(FULL, vc, k);
-                s1 += tile[(k + 1) * TILE + lane] * __shfl_sync(FULL, vc, k + 1);
-            }
-            v[TILE * J + lane] = s0 + s1;
-        }
-        __syncthreads();
-    }
     double dot = 0.0;
-    for (int e = e0 + threadIdx.x; e < e1; e += blockDim.x) {
+    for (int e = e0 + rank * blockDim.x + threadIdx.x; e < e1; e += C * blockDim.x) {
         const double yv = rsign[e] * v[pos[rdof[e] - o]];
         if (MODE == 1) {
             out[e] = yv;
@@ -2014,6 +2091,9 @@ struct GpuSolver::Impl {
     // device K^+ and the right-hand-side / primal vectors
     KplusDev KP{};
     long long kplus_tiles_kept = 0, kplus_tiles_total = 0;   // factor tiles applied / stored
+    int kp_cluster = 1;                                       // CTAs per subdomain of the K^+ sweeps
+    KpSmem kp_smem{0, 0};
+    size_t kp_smem_bytes = 0;
     long long kp_tsum = 0;                                    // 32-blocks of all subdomains
     double *kp_gvec = nullptr;                                // kplus_mma_kernel<NC, true> vectors
     size_t kp_gvec_n = 0;
@@ -2145,6 +2225,7 @@ struct GpuSolver::Impl {
 
 // dynamic shared memory available to kplus_multi_kernel<NC> next to its static partial sums
 static size_t kplus_multi_smem(int nc) { return (size_t)220 * 1024 - (size_t)nc * 8 * TILE * sizeof(double); }
+constexpr size_t KP_SMEM_MAX = (size_t)224 * 1024;   // dynamic shared memory of the K^+ sweeps, at most
 // dynamic shared memory available to kplus_mma_kernel<NC> next to its 16 KB per 8 columns of partials
 static size_t kplus_mma_smem(int nc) { return (size_t)226 * 1024 - (size_t)(nc / 8) * 16 * 1024; }
 static bool kplus_mma_enabled() {
@@ -2203,9 +2284,8 @@ void GpuSolver::Impl::launch_kplus_multi(const double *in, double *out, int ncol
 }
 
 void GpuSolver::Impl::launch_kplus(const double *in, double *out, int mode) {
-    size_t sm = sizeof(double) * TILE * (size_t)max_T;
-    kplus_kernel<<<P.nd, 256, sm, stream>>>(KP, in, out, mode);
-    CUDA_CHECK(cudaGetLastError());
+    launch_cluster(kplus_kernel, kp_cluster, dim3(P.nd * kp_cluster), dim3(KP_WARPS * 32), kp_smem_bytes, stream, KP, in,
+                   out, mode, kp_smem);
 }
 
 void GpuSolver::Impl::upload_kplus(const Decomposition &dec, const Prep &prep, const std::vector<int> &loff,
@@ -2340,6 +2420,48 @@ void GpuSolver::Impl::upload_kplus(const Decomposition &dec, const Prep &prep, c
         for (int d = 0; d < nd; ++d) tpre[d + 1] = tpre[d] + tn[d];
         KP.tpre = upload(tpre);
         kp_tsum = tpre[nd];
+        // the nonzero tiles as symmetric bit rows, the subdomains by descending work
+        std::vector<int> mw(nd), order(nd);
+        std::vector<long long> moff(nd + 1, 0), work(nd);
+        long long wsum = 0, wmax = 0;
+        int mask_max = 0;
+        for (int d = 0; d < nd; ++d) {
+            mw[d] = (tn[d] + 31) / 32;
+            moff[d + 1] = moff[d] + (long long)tn[d] * mw[d];
+            mask_max = std::max(mask_max, tn[d] * mw[d]);
+            work[d] = cptr[cbase[d] + tn[d]] - cptr[cbase[d]];
+            wsum += work[d];
+            wmax = std::max(wmax, work[d]);
+            order[d] = d;
+        }
+        std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return work[a] > work[b]; });
+        std::vector<unsigned> mask((size_t)moff[nd], 0u);
+        for (int d = 0; d < nd; ++d) {
+            unsigned *m = mask.data() + moff[d];
+            for (int J = 0; J < tn[d]; ++J)
+                for (int q = cptr[cbase[d] + J]; q < cptr[cbase[d] + J + 1]; ++q) {
+                    const int I = rows[q];
+                    m[(size_t)J * mw[d] + (I >> 5)] |= 1u << (I & 31);
+                    m[(size_t)I * mw[d] + (J >> 5)] |= 1u << (J & 31);
+                }
+        }
+        KP.mw = upload(mw);
+        KP.moff = upload(moff);
+        KP.mask = upload(mask);
+        KP.order = upload(order);
+        // Cluster size: enough CTAs for two per SM, and the largest subdomain's share of the work
+        // within the share of one SM; at least eight blocks per CTA.
+        kp_cluster = 1;
+        while (kp_cluster < 8 && max_T >= 16 * kp_cluster &&
+               (2 * kp_cluster * nd <= 2 * nsm || wmax * nsm > wsum * kp_cluster))
+            kp_cluster *= 2;
+        const size_t vb = sizeof(double) * TILE * (size_t)max_T, db = sizeof(double) * KP_WARPS * TILE * TILE,
+                     mb = sizeof(unsigned) * (size_t)mask_max;
+        kp_smem.vblocks = max_T;
+        kp_smem.parts = 0;
+        kp_smem_bytes = vb;
+        if (kp_smem_bytes + db <= KP_SMEM_MAX) { kp_smem.parts |= KPS_DIAG; kp_smem_bytes += db; }
+        if (kp_smem_bytes + mb <= KP_SMEM_MAX) { kp_smem.parts |= KPS_MASK; kp_smem_bytes += mb; }
         kplus_tiles_kept = kept;
         kplus_tiles_total = ntiles;
     }
@@ -2364,9 +2486,9 @@ void GpuSolver::Impl::upload_kplus(const Decomposition &dec, const Prep &prep, c
     d_g = alloc<double>(ntot);
     d_rhs = alloc<double>(std::max(1, n_caller));
     d_sol = alloc<double>(std::max(1, n_caller));
-    cudaFuncSetAttribute(kplus_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-    cudaFuncSetAttribute(kplus_dual_kernel<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-    cudaFuncSetAttribute(kplus_dual_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+    CUDA_CHECK(cudaFuncSetAttribute(kplus_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)KP_SMEM_MAX));
+    CUDA_CHECK(cudaFuncSetAttribute(kplus_dual_kernel<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)KP_SMEM_MAX));
+    CUDA_CHECK(cudaFuncSetAttribute(kplus_dual_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)KP_SMEM_MAX));
     CUDA_CHECK(cudaFuncSetAttribute(kplus_multi_kernel<16>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kplus_multi_smem(16)));
     CUDA_CHECK(cudaFuncSetAttribute(kplus_multi_kernel<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kplus_multi_smem(8)));
     CUDA_CHECK(cudaFuncSetAttribute(kplus_multi_kernel<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kplus_multi_smem(4)));
@@ -2739,14 +2861,8 @@ void GpuSolver::Impl::release(void *p) {
 
 void GpuSolver::Impl::launch_implicit(int mode, const double *src, const double *src2, double *out, int slot) {
     FETI_CHECK(mode == 0 || mode == 1, "internal: implicit F apply in an unsupported mode");
-    const size_t sm = sizeof(double) * TILE * (size_t)max_T;
-    if (mode == 0)
-        launch_pdl(kplus_dual_kernel<0>, dim3(P.nd), dim3(256), sm, stream, KP, P, (const int *)d_rdof,
-                   (const double *)d_rsign, src, src2, out, slot);
-    else
-        launch_pdl(kplus_dual_kernel<1>, dim3(P.nd), dim3(256), sm, stream, KP, P, (const int *)d_rdof,
-                   (const double *)d_rsign, src, src2, out, slot);
-    CUDA_CHECK(cudaGetLastError());
+    launch_cluster(mode == 0 ? kplus_dual_kernel<0> : kplus_dual_kernel<1>, kp_cluster, dim3(P.nd * kp_cluster),
+                   dim3(KP_WARPS * 32), kp_smem_bytes, stream, KP, P, d_rdof, d_rsign, src, src2, out, slot, kp_smem);
 }
 
 void GpuSolver::Impl::launch_tiles(const TileSetHost &T, int mode, const double *src, const double *src2, double *out,
@@ -3157,7 +3273,8 @@ void GpuSolver::upload(const Decomposition &dec, const Prep &prep, const SolveOp
     P.alpha = I.alloc<double>(prep.n_kern + KS);
     CUDA_CHECK(cudaMemset(P.alpha, 0, sizeof(double) * (prep.n_kern + KS)));
     I.e_dev = I.alloc<double>(P.nP);
-    P.part_w = I.alloc<double>(2 * nd); P.part_rho = I.alloc<double>(nd); P.part_b = I.alloc<double>(nd);
+    P.part_w = I.alloc<double>(9 * (size_t)nd);   // the second part: up to 8 CTAs per subdomain (implicit F)
+    P.part_rho = I.alloc<double>(nd); P.part_b = I.alloc<double>(nd);
     P.rho_hist = I.alloc<double>((size_t)opt.max_iterations + 64);
     I.st = I.alloc<DevState>(1);
     P.st = I.st;
