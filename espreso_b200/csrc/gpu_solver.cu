@@ -1498,131 +1498,15 @@ __global__ void __launch_bounds__(KP_WARPS * 32, 2) kplus_dual_kernel(KplusDev K
     if (MODE == 1) grid_total(block_sum(dot, sh), P.part_w + P.nd, P.done + DONE_PAP_IMPLICIT, P.scal + SC_PAP, sh);
 }
 
-// K^+ on NC right-hand sides at once (columns j0 .. j0+NC-1 of in/out, `stride` doubles apart):
-// every factor tile is loaded once per pass and applied to all NC columns, so the factor is read
-// once for NC load cases.  Same tile walk and modes as kplus_kernel; z (mode 1/2) holds the
-// forward results of every column at the same stride.  Warps take off-diagonal tiles; warp w
-// handles the diagonal blocks of columns w, w + 8, ...
-template <int NC>
-__global__ void __launch_bounds__(256) kplus_multi_kernel(KplusDev K, const double *in, double *out, int mode,
-                                                          int j0, long long stride, double *z) {
-    extern __shared__ double vm[];              // [NC][TILE * T]
-    __shared__ double part[8][NC][TILE];
-    const int d = blockIdx.x;
-    const int n = K.n[d], T = K.tn[d], o = K.doff[d];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-    const int NP = TILE * T;
-    const int *pos = K.pos + o;
-    const uint4 *tiles = reinterpret_cast<const uint4 *>(K.L) + (size_t)K.tile0[d] * (TILE * 16);
-    const double *dtiles = K.L + (size_t)K.tile0[d] * TILE * TILE;
-    const int *cp = K.cptr + K.cbase[d];
-    const int jt = mode == KPLUS_FULL ? 0 : K.jt[d];
-    for (int i = threadIdx.x; i < NC * NP; i += blockDim.x) vm[i] = 0.0;
-    __syncthreads();
-    for (int c = 0; c < NC; ++c)
-        for (int i = threadIdx.x; i < n; i += blockDim.x) vm[c * NP + pos[i]] = in[(size_t)(j0 + c) * stride + o + i];
-    __syncthreads();
-    const int cq = lane % 16, h = lane / 16, idx = 2 * cq + h;
-    for (int J = (mode == KPLUS_PRIMAL ? jt : 0); J < T; ++J) {
-        {
-            const double *row = dtiles + (size_t)ltile(T, J, J) * TILE * TILE + lane * TILE;
-            for (int c = warp; c < NC; c += nw) {
-                double *vc = vm + c * NP;
-                const double vr = vc[TILE * J + lane];
-                double s0 = 0.0, s1 = 0.0;
-#pragma unroll
-                for (int k = 0; k < TILE; k += 2) {
-                    s0 += row[k] * __shfl_sync(FULL, vr, k);
-                    s1 += row[k + 1] * __shfl_sync(FULL, vr, k + 1);
-                }
-                vc[TILE * J + lane] = s0 + s1;
-            }
-        }
-        __syncthreads();
-        for (int qi = cp[J] + 1 + warp; qi < cp[J + 1]; qi += nw) {
-            const int I = K.rows[qi];
-            const uint4 *tp = tiles + (size_t)ltile(T, I, J) * (TILE * 16);
-            uint4 t[16];
-#pragma unroll
-            for (int q = 0; q < 16; ++q) t[q] = ld_stream(tp + q * 32 + lane);
-            for (int c = 0; c < NC; ++c) {
-                double *vc = vm + c * NP;
-                const double x0 = vc[TILE * J + 2 * cq], x1 = vc[TILE * J + 2 * cq + 1];
-                double rs[16];
-#pragma unroll
-                for (int q = 0; q < 16; ++q)
-                    rs[q] = __hiloint2double(t[q].y, t[q].x) * x0 + __hiloint2double(t[q].w, t[q].z) * x1;
-                const double r = reduce_scatter<16, 0>(rs, lane);
-                vc[TILE * I + idx] -= r;
-            }
-        }
-        __syncthreads();
-    }
-    if (mode == KPLUS_TOUCHED) {
-        for (int c = 0; c < NC; ++c)
-            for (int i = threadIdx.x; i < n; i += blockDim.x) z[(size_t)(j0 + c) * stride + o + i] = vm[c * NP + i];
-        __syncthreads();
-    } else if (mode == KPLUS_PRIMAL) {
-        for (int c = 0; c < NC; ++c)
-            for (int i = threadIdx.x; i < n; i += blockDim.x) vm[c * NP + i] += z[(size_t)(j0 + c) * stride + o + i];
-        __syncthreads();
-    }
-    for (int J = T - 1; J >= (mode == KPLUS_TOUCHED ? jt : 0); --J) {
-        double cpart[NC];
-#pragma unroll
-        for (int c = 0; c < NC; ++c) cpart[c] = 0.0;
-        for (int qi = cp[J] + 1 + warp; qi < cp[J + 1]; qi += nw) {
-            const int I = K.rows[qi];
-            const uint4 *tp = tiles + (size_t)ltile(T, I, J) * (TILE * 16);
-            uint4 t[16];
-#pragma unroll
-            for (int q = 0; q < 16; ++q) t[q] = ld_stream(tp + q * 32 + lane);
-#pragma unroll
-            for (int c = 0; c < NC; ++c) {
-                const double *vc = vm + c * NP;
-                double cs[2] = {0.0, 0.0};
-#pragma unroll
-                for (int q = 0; q < 16; ++q) {
-                    const double xr = vc[TILE * I + 2 * q + h];
-                    cs[0] += __hiloint2double(t[q].y, t[q].x) * xr;
-                    cs[1] += __hiloint2double(t[q].w, t[q].z) * xr;
-                }
-                cpart[c] += reduce_scatter<2, 4>(cs, lane);
-            }
-        }
-#pragma unroll
-        for (int c = 0; c < NC; ++c) part[warp][c][idx] = cpart[c];
-        __syncthreads();
-        {
-            const double *tile = dtiles + (size_t)ltile(T, J, J) * TILE * TILE;
-            for (int c = warp; c < NC; c += nw) {
-                double *vc = vm + c * NP;
-                double v0 = vc[TILE * J + lane];
-                for (int w = 0; w < nw; ++w) v0 -= part[w][c][lane];
-                double s0 = 0.0, s1 = 0.0;
-#pragma unroll
-                for (int k = 0; k < TILE; k += 2) {
-                    s0 += tile[k * TILE + lane] * __shfl_sync(FULL, v0, k);
-                    s1 += tile[(k + 1) * TILE + lane] * __shfl_sync(FULL, v0, k + 1);
-                }
-                vc[TILE * J + lane] = s0 + s1;
-            }
-        }
-        __syncthreads();
-    }
-    for (int c = 0; c < NC; ++c)
-        for (int i = threadIdx.x; i < n; i += blockDim.x) out[(size_t)(j0 + c) * stride + o + i] = vm[c * NP + pos[i]];
-}
-
-// K^+ on NC = 8 or 16 right-hand sides with FP64 tensor-core MMAs (mma.m8n8k4.f64).  Same tile
-// walk, nonzero-tile lists and modes as kplus_multi_kernel.  Every 32 x 32 step is
-// C(32 x NC) += A(32 x 32) B(32 x NC) as 4 x NC/8 blocks of 8 x 8 over 8 k-steps of 4: A is the
-// factor tile read straight from global memory in fragment order (the tile in the forward pass, its
-// transpose in the backward pass; every 32-byte sector is read once), B the column block of the
-// vectors in shared memory.  The vectors are kept in factor order, NP + KPM_PAD doubles apart, so
-// that the fragment loads and stores take the minimum two wavefronts.  Warps take the off-diagonal
-// tiles of a block column in turn; the diagonal step (inverse diagonal tile) is split over 4 x NC/8
-// warps.  The backward partial sums of the warps meet in shared memory.
+// K^+ on NC = 8 or 16 right-hand sides (columns j0 .. j0+NC-1 of in/out, `stride` doubles apart; columns
+// from nact on are zero and not stored) with FP64 tensor-core MMAs (mma.m8n8k4.f64): every factor
+// tile is read once per pass for NC load cases.  The sweep is kp_sweep's: step s publishes its solved
+// 32 x NC block to the cluster, the target blocks are dealt to the warps, the owner of block s + 1 goes
+// ahead.  Every 32 x 32 step is C(32 x NC) += A(32 x 32) B(32 x NC) as 4 x NC/8 blocks of 8 x 8 over 8
+// k-steps of 4: A is the factor tile read straight from global memory in fragment order (the tile in the
+// forward pass, its transpose in the backward pass; every 32-byte sector is read once), B the column
+// block of the vectors.  The vectors are kept in factor order, NP + KPM_PAD doubles apart, so that the
+// fragment loads and stores take the minimum two wavefronts.
 constexpr int KPM_PAD = 4;
 
 __device__ __forceinline__ void dmma84(double (&c)[2], double a, double b) {
@@ -1631,176 +1515,182 @@ __device__ __forceinline__ void dmma84(double (&c)[2], double a, double b) {
                  : "d"(a), "d"(b));
 }
 
-template <int NC, bool GL>
-__global__ void __launch_bounds__(256, 1) kplus_mma_kernel(KplusDev K, const double *in, double *out, int mode,
-                                                           int j0, long long stride, double *z, double *gvec) {
-    static_assert(NC == 8 || NC == 16, "K+ MMA kernel: 8 or 16 columns");
+// One triangular sweep on NC columns (kp_sweep with MMAs).  GL: vm is one global array shared by the
+// cluster's CTAs (the cluster barriers order it), else every CTA's own copy in shared memory.
+template <int NC, bool GL, bool FWD>
+__device__ void kpm_sweep(const double *L, const unsigned *mask, int mw, int T, int lo, double *vm, int NPp) {
     constexpr int NB = NC / 8;
-    extern __shared__ double vm_s[];               // [NC][NP + KPM_PAD]
-    __shared__ double part[8][4 * NB * 2 * 32];    // backward partials per warp, fragment order
-    const int d = blockIdx.x;
-    const int n = K.n[d], T = K.tn[d], o = K.doff[d];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int gr = lane >> 2, gc = lane & 3;       // fragment row (group) and column in the group
-    const int NP = TILE * T, NPp = NP + KPM_PAD;
-    const int *pos = K.pos + o;
-    const double *L = K.L + (size_t)K.tile0[d] * TILE * TILE;
-    const int *cp = K.cptr + K.cbase[d];
-    const int jt = mode == KPLUS_FULL ? 0 : K.jt[d];
-    // GL: the vectors of subdomains too large for shared memory live in a global (L2-resident)
-    // scratch, NC (32 T_d + KPM_PAD) doubles per subdomain; the block barriers order them as well
-    double *vm = GL ? gvec + (size_t)NC * ((size_t)TILE * K.tpre[d] + (size_t)KPM_PAD * d) : vm_s;
-    for (int i = threadIdx.x; i < NC * NPp; i += blockDim.x) vm[i] = 0.0;
-    __syncthreads();
-    for (int c = 0; c < NC; ++c)
-        for (int i = threadIdx.x; i < n; i += blockDim.x) vm[c * NPp + pos[i]] = in[(size_t)(j0 + c) * stride + o + i];
-    __syncthreads();
-
-    // block J := inv(L_JJ) block J (trans: inv(L_JJ)^T), warps 0 .. 4 NB - 1, one 8 x 8 block each
-    auto diag = [&](int J, bool trans) {
-        const bool act = warp < 4 * NB;
-        const int mb = warp & 3, nb = warp >> 2;
-        double acc[2] = {0.0, 0.0};
-        if (act) {
-            const double *tile = L + (size_t)ltile(T, J, J) * TILE * TILE;
-            const double *bcol = vm + (size_t)(8 * nb + gr) * NPp + TILE * J;
-#pragma unroll
-            for (int ks = 0; ks < 8; ++ks) {
-                const int k = 4 * ks + gc;
-                const double a = trans ? __ldg(tile + k * TILE + 8 * mb + gr) : __ldg(tile + (8 * mb + gr) * TILE + k);
-                dmma84(acc, a, bcol[k]);
-            }
-        }
-        __syncthreads();   // block J read by every active warp before it is overwritten
-        if (act) {
-            double *cc = vm + (size_t)(8 * nb + 2 * gc) * NPp + TILE * J + 8 * mb + gr;
-            cc[0] = acc[0];
-            cc[NPp] = acc[1];
-        }
-        __syncthreads();
-    };
-
-    // Factor fragments come straight from global memory in fragment order; a warp's next tile is
-    // loaded while the MMAs of its current one run, and its first tile of the next block column
-    // before the barriers and the diagonal step of that column.
-    auto fload = [&](int J, int qx, double (&a)[4][8]) {
-        const double *tile = L + (size_t)ltile(T, K.rows[qx], J) * TILE * TILE + gr * TILE + gc;
+    const int C = (int)cluster_size_x(), NW = KP_WARPS * C, W = warp * C + (int)cluster_rank_x();
+    const int steps = T - lo;
+    if (steps <= 0) return;   // the same for the whole cluster
+    auto blk = [&](int s) { return FWD ? lo + s : T - 1 - s; };
+    auto aload = [&](int s, int t, double (&a)[4][8]) {   // A of the tile coupling steps s <= t
+        const int x = blk(s), y = blk(t);
+        const double *tp = L + (size_t)(FWD ? ltile(T, y, x) : ltile(T, x, y)) * TILE * TILE;
 #pragma unroll
         for (int mb = 0; mb < 4; ++mb)
 #pragma unroll
-            for (int ks = 0; ks < 8; ++ks) a[mb][ks] = __ldg(tile + 8 * mb * TILE + 4 * ks);
+            for (int ks = 0; ks < 8; ++ks)
+                a[mb][ks] = FWD ? __ldg(tp + (8 * mb + gr) * TILE + 4 * ks + gc) : __ldg(tp + (4 * ks + gc) * TILE + 8 * mb + gr);
     };
-    auto bload = [&](int J, int qx, double (&a)[4][8]) {   // A = L_IJ^T: A[m][k] = L_IJ[k][m]
-        const double *tile = L + (size_t)ltile(T, K.rows[qx], J) * TILE * TILE + gc * TILE + gr;
-#pragma unroll
-        for (int mb = 0; mb < 4; ++mb)
-#pragma unroll
-            for (int ks = 0; ks < 8; ++ks) a[mb][ks] = __ldg(tile + 4 * ks * TILE + 8 * mb);
-    };
-    double a0[4][8], a1[4][8];
-    // forward: L y = f
-    const int jf = mode == KPLUS_PRIMAL ? jt : 0;
-    if (jf < T && cp[jf] + 1 + warp < cp[jf + 1]) fload(jf, cp[jf] + 1 + warp, a0);
-    for (int J = jf; J < T; ++J) {
-        diag(J, false);
-        double bf[8][NB];
+    auto bload = [&](int t, double (&b)[8][NB]) {
 #pragma unroll
         for (int ks = 0; ks < 8; ++ks)
 #pragma unroll
-            for (int nb = 0; nb < NB; ++nb) bf[ks][nb] = vm[(size_t)(8 * nb + gr) * NPp + TILE * J + 4 * ks + gc];
-        auto fproc = [&](int qx, const double (&af)[4][8]) {
-            const int I = K.rows[qx];
-            double acc[4][NB][2];
-#pragma unroll
-            for (int mb = 0; mb < 4; ++mb)
-#pragma unroll
-                for (int nb = 0; nb < NB; ++nb) {
-                    acc[mb][nb][0] = 0.0;
-                    acc[mb][nb][1] = 0.0;
-#pragma unroll
-                    for (int ks = 0; ks < 8; ++ks) dmma84(acc[mb][nb], af[mb][ks], bf[ks][nb]);
-                }
-#pragma unroll
-            for (int mb = 0; mb < 4; ++mb)
-#pragma unroll
-                for (int nb = 0; nb < NB; ++nb) {
-                    double *cc = vm + (size_t)(8 * nb + 2 * gc) * NPp + TILE * I + 8 * mb + gr;
-                    cc[0] -= acc[mb][nb][0];
-                    cc[NPp] -= acc[mb][nb][1];
-                }
-        };
-        const int qe = cp[J + 1];
-        for (int qi = cp[J] + 1 + warp; qi < qe; qi += 16) {
-            if (qi + 8 < qe) fload(J, qi + 8, a1);
-            fproc(qi, a0);
-            if (qi + 8 >= qe) break;
-            if (qi + 16 < qe) fload(J, qi + 16, a0);
-            fproc(qi + 8, a1);
-        }
-        if (J + 1 < T && cp[J + 1] + 1 + warp < cp[J + 2]) fload(J + 1, cp[J + 1] + 1 + warp, a0);
-        __syncthreads();
-    }
-    if (mode == KPLUS_TOUCHED) {
-        for (int c = 0; c < NC; ++c)
-            for (int i = threadIdx.x; i < n; i += blockDim.x) z[(size_t)(j0 + c) * stride + o + i] = vm[c * NPp + i];
-        __syncthreads();
-    } else if (mode == KPLUS_PRIMAL) {
-        for (int c = 0; c < NC; ++c)
-            for (int i = threadIdx.x; i < n; i += blockDim.x) vm[c * NPp + i] += z[(size_t)(j0 + c) * stride + o + i];
-        __syncthreads();
-    }
-    // backward: L^T x = y (mode 1: down to block jt)
-    const int jb = mode == KPLUS_TOUCHED ? jt : 0;
-    if (T - 1 >= jb && cp[T - 1] + 1 + warp < cp[T]) bload(T - 1, cp[T - 1] + 1 + warp, a0);
-    for (int J = T - 1; J >= jb; --J) {
-        double acc[4][NB][2];
+            for (int nb = 0; nb < NB; ++nb) b[ks][nb] = vm[(size_t)(8 * nb + gr) * NPp + TILE * blk(t) + 4 * ks + gc];
+    };
+    auto mult = [&](const double (&a)[4][8], const double (&b)[8][NB], double (&c)[4][NB][2]) {
 #pragma unroll
         for (int mb = 0; mb < 4; ++mb)
 #pragma unroll
-            for (int nb = 0; nb < NB; ++nb) acc[mb][nb][0] = acc[mb][nb][1] = 0.0;
-        auto bproc = [&](int qx, const double (&af)[4][8]) {
-            const int I = K.rows[qx];
-            double bf[8][NB];
+            for (int nb = 0; nb < NB; ++nb) c[mb][nb][0] = c[mb][nb][1] = 0.0;
 #pragma unroll
-            for (int ks = 0; ks < 8; ++ks)
-#pragma unroll
-                for (int nb = 0; nb < NB; ++nb) bf[ks][nb] = vm[(size_t)(8 * nb + gr) * NPp + TILE * I + 4 * ks + gc];
+        for (int ks = 0; ks < 8; ++ks)
 #pragma unroll
             for (int mb = 0; mb < 4; ++mb)
 #pragma unroll
-                for (int nb = 0; nb < NB; ++nb)
-#pragma unroll
-                    for (int ks = 0; ks < 8; ++ks) dmma84(acc[mb][nb], af[mb][ks], bf[ks][nb]);
-        };
-        const int qe = cp[J + 1];
-        for (int qi = cp[J] + 1 + warp; qi < qe; qi += 16) {
-            if (qi + 8 < qe) bload(J, qi + 8, a1);
-            bproc(qi, a0);
-            if (qi + 8 >= qe) break;
-            if (qi + 16 < qe) bload(J, qi + 16, a0);
-            bproc(qi + 8, a1);
-        }
-        if (J - 1 >= jb && cp[J - 1] + 1 + warp < cp[J]) bload(J - 1, cp[J - 1] + 1 + warp, a0);
+                for (int nb = 0; nb < NB; ++nb) dmma84(c[mb][nb], a[mb][ks], b[ks][nb]);
+    };
+    auto cell = [&](int t, int mb, int nb) { return vm + (size_t)(8 * nb + 2 * gc) * NPp + TILE * blk(t) + 8 * mb + gr; };
+    auto subtract = [&](int t, const double (&a)[4][8], const double (&b)[8][NB]) {
+        double c[4][NB][2];
+        mult(a, b, c);
 #pragma unroll
         for (int mb = 0; mb < 4; ++mb)
 #pragma unroll
             for (int nb = 0; nb < NB; ++nb) {
-                part[warp][((mb * NB + nb) * 2 + 0) * 32 + lane] = acc[mb][nb][0];
-                part[warp][((mb * NB + nb) * 2 + 1) * 32 + lane] = acc[mb][nb][1];
+                double *p = cell(t, mb, nb);
+                p[0] -= c[mb][nb][0];
+                p[NPp] -= c[mb][nb][1];
             }
-        __syncthreads();
-        for (int q = threadIdx.x; q < 32 * NC; q += blockDim.x) {
-            const int ln = q & 31, e = (q >> 5) & 1, blk = q >> 6, mb = blk / NB, nb = blk % NB;
-            double sum = 0.0;
+    };
+    auto publish = [&](int s, const double (&a)[4][8]) {   // a: the diagonal tile of step s
+        double b[8][NB], c[4][NB][2];
+        __syncwarp();
+        bload(s, b);
+        mult(a, b, c);
+        __syncwarp();
 #pragma unroll
-            for (int w = 0; w < 8; ++w) sum += part[w][q];
-            vm[(size_t)(8 * nb + 2 * (ln & 3) + e) * NPp + TILE * J + 8 * mb + (ln >> 2)] -= sum;
-        }
-        __syncthreads();
-        diag(J, true);
+        for (int mb = 0; mb < 4; ++mb)
+#pragma unroll
+            for (int nb = 0; nb < NB; ++nb) {
+                double *p = cell(s, mb, nb);
+                if (GL) {
+                    p[0] = c[mb][nb][0];
+                    p[NPp] = c[mb][nb][1];
+                } else {
+                    for (int r = 0; r < C; ++r) {
+                        st_cluster(p, (unsigned)r, c[mb][nb][0]);
+                        st_cluster(p + NPp, (unsigned)r, c[mb][nb][1]);
+                    }
+                }
+            }
+    };
+    double a0[4][8], a1[4][8];
+    if (W == 0) {
+        aload(0, 0, a0);
+        publish(0, a0);
     }
-    for (int c = 0; c < NC; ++c)
-        for (int i = threadIdx.x; i < n; i += blockDim.x) out[(size_t)(j0 + c) * stride + o + i] = vm[c * NPp + pos[i]];
+    cluster_arrive();
+    for (int s = 0; s < steps; ++s) {
+        const unsigned *mrow = mask + (size_t)blk(s) * mw;
+        int t = s + 1 + (W - (s + 1) % NW + NW) % NW;
+        const bool crit = t == s + 1 && t < steps;
+        auto next = [&](int u) {
+            while (u < steps && !((__ldg(mrow + (blk(u) >> 5)) >> (blk(u) & 31)) & 1u)) u += NW;
+            return u;
+        };
+        t = next(t);
+        // the loads that do not depend on block s: the first tile, and the diagonal tile or the second one
+        int t2 = steps;
+        if (crit) {
+            if (t == s + 1) aload(s, t, a0);
+            aload(s + 1, s + 1, a1);
+        } else if (t < steps) {
+            aload(s, t, a0);
+            t2 = next(t + NW);
+        }
+        cluster_wait();                                    // block s is solved
+        double b[8][NB];
+        if (crit) {
+            if (t == s + 1) {
+                bload(s, b);
+                subtract(t, a0, b);
+                t = next(t + NW);
+            }
+            publish(s + 1, a1);
+            cluster_arrive();
+            if (t < steps) {
+                aload(s, t, a0);
+                t2 = next(t + NW);
+            }
+        } else if (s + 1 < steps) {
+            cluster_arrive();
+        }
+        if (t >= steps) continue;
+        bload(s, b);
+        for (;;) {
+            if (t2 < steps) aload(s, t2, a1);
+            subtract(t, a0, b);
+            if (t2 >= steps) break;
+            t = next(t2 + NW);
+            if (t < steps) aload(s, t, a0);
+            subtract(t2, a1, b);
+            if (t >= steps) break;
+            t2 = next(t + NW);
+        }
+    }
+}
+
+template <int NC, bool GL>
+__global__ void __launch_bounds__(KP_WARPS * 32, 1) kplus_mma_kernel(KplusDev K, const double *in, double *out,
+                                                                     int mode, int j0, int nact, long long stride,
+                                                                     double *z, double *gvec) {
+    static_assert(NC == 8 || NC == 16, "K+ MMA kernel: 8 or 16 columns");
+    pdl_enter();
+    extern __shared__ double vm_s[];               // [NC][NP + KPM_PAD]
+    const int C = (int)cluster_size_x(), rank = (int)cluster_rank_x();
+    const int d = K.order[blockIdx.x / C];
+    const int n = K.n[d], T = K.tn[d], o = K.doff[d];
+    const int NPp = TILE * T + KPM_PAD;
+    const int *pos = K.pos + o;
+    const double *L = K.L + (size_t)K.tile0[d] * TILE * TILE;
+    const unsigned *mask = K.mask + K.moff[d];
+    const int jt = mode == KPLUS_FULL ? 0 : K.jt[d];
+    // GL: the vectors of subdomains too large for shared memory live in a global (L2-resident)
+    // scratch, NC (32 T_d + KPM_PAD) doubles per subdomain, which the cluster's CTAs share
+    double *vm = GL ? gvec + (size_t)NC * ((size_t)TILE * K.tpre[d] + (size_t)KPM_PAD * d) : vm_s;
+    // rows of the vectors this CTA fills: all of its own copy, or its share of the common one
+    const int i0 = GL ? rank * blockDim.x + threadIdx.x : threadIdx.x, di = GL ? C * blockDim.x : blockDim.x;
+    const int s0 = rank * blockDim.x + threadIdx.x, ds = C * blockDim.x;
+    for (int i = i0; i < NC * NPp; i += di) vm[i] = 0.0;
+    cluster_arrive();
+    cluster_wait();
+    for (int c = 0; c < nact; ++c)
+        for (int i = i0; i < n; i += di) vm[(size_t)c * NPp + pos[i]] = in[(size_t)(j0 + c) * stride + o + i];
+    cluster_arrive();
+    cluster_wait();
+    // forward: L y = f
+    kpm_sweep<NC, GL, true>(L, mask, K.mw[d], T, mode == KPLUS_PRIMAL ? jt : 0, vm, NPp);
+    cluster_arrive();
+    cluster_wait();
+    if (mode == KPLUS_TOUCHED) {
+        for (int c = 0; c < nact; ++c)
+            for (int i = s0; i < n; i += ds) z[(size_t)(j0 + c) * stride + o + i] = vm[(size_t)c * NPp + i];
+    } else if (mode == KPLUS_PRIMAL) {
+        for (int c = 0; c < nact; ++c)
+            for (int i = i0; i < n; i += di) vm[(size_t)c * NPp + i] += z[(size_t)(j0 + c) * stride + o + i];
+    }
+    cluster_arrive();
+    cluster_wait();
+    // backward: L^T x = y (mode 1: down to block jt)
+    kpm_sweep<NC, GL, false>(L, mask, K.mw[d], T, mode == KPLUS_TOUCHED ? jt : 0, vm, NPp);
+    cluster_arrive();
+    cluster_wait();
+    for (int c = 0; c < nact; ++c)
+        for (int i = s0; i < n; i += ds) out[(size_t)(j0 + c) * stride + o + i] = vm[(size_t)c * NPp + pos[i]];
 }
 
 // subdomain loads f_i = rhs(caller DOF) / multiplicity
@@ -2224,62 +2114,38 @@ struct GpuSolver::Impl {
 };
 
 // dynamic shared memory available to kplus_multi_kernel<NC> next to its static partial sums
-static size_t kplus_multi_smem(int nc) { return (size_t)220 * 1024 - (size_t)nc * 8 * TILE * sizeof(double); }
 constexpr size_t KP_SMEM_MAX = (size_t)224 * 1024;   // dynamic shared memory of the K^+ sweeps, at most
-// dynamic shared memory available to kplus_mma_kernel<NC> next to its 16 KB per 8 columns of partials
-static size_t kplus_mma_smem(int nc) { return (size_t)226 * 1024 - (size_t)(nc / 8) * 16 * 1024; }
-static bool kplus_mma_enabled() {
-    static const bool on = [] {
-        const char *e = getenv("FETI4I_KPLUS_MMA");
-        return !(e && e[0] == '0');
-    }();
-    return on;
-}
 
-// K^+ on ncol columns (stride ntot): groups of NC columns per pass, NC as large as shared memory allows.
+// K^+ on ncol columns (stride ntot): up to 16 columns per pass over the factor, as many as shared memory
+// holds; beyond that (T > 108 blocks) 16 with the vectors in global memory.  A group of fewer columns
+// runs padded, which costs less than another pass; a single column takes the one-vector kernel.
 void GpuSolver::Impl::launch_kplus_multi(const double *in, double *out, int ncol, int mode, double *z) {
-    const size_t per_col = sizeof(double) * TILE * (size_t)max_T;
-    int j0 = 0;
-    while (j0 < ncol) {
+    auto smem = [&](int nc) { return sizeof(double) * (size_t)nc * ((size_t)TILE * max_T + KPM_PAD); };
+    for (int j0 = 0; j0 < ncol;) {
         const int left = ncol - j0;
-        // (groups of 16, 8, 4 and 2 gave 120, 128, 120 and 133 ms of batched e2e on c2)
-        int nc = 16;
-        while (nc > 1 && (nc > left || (size_t)nc * per_col > kplus_multi_smem(nc))) nc /= 2;
-        const size_t sm = (size_t)nc * per_col;
-        // FP64 tensor-core variant for 8 or 16 columns when the padded vectors fit next to its
-        // partial sums
-        const size_t sm_mma = sizeof(double) * (size_t)nc * ((size_t)TILE * max_T + KPM_PAD);
-        if (kplus_mma_enabled() && (nc == 16 || nc == 8) && sm_mma <= kplus_mma_smem(nc)) {
-            if (nc == 16) kplus_mma_kernel<16, false><<<P.nd, 256, sm_mma, stream>>>(KP, in, out, mode, j0, ntot, z, nullptr);
-            else kplus_mma_kernel<8, false><<<P.nd, 256, sm_mma, stream>>>(KP, in, out, mode, j0, ntot, z, nullptr);
-            CUDA_CHECK(cudaGetLastError());
-            j0 += nc;
-            continue;
+        if (left == 1) {
+            const size_t o = (size_t)j0 * ntot;
+            KplusDev K1 = KP;
+            if (z) K1.z = z + o;
+            launch_cluster(kplus_kernel, kp_cluster, dim3(P.nd * kp_cluster), dim3(KP_WARPS * 32), kp_smem_bytes, stream,
+                           K1, in + o, out + o, mode, kp_smem);
+            return;
         }
-        if (kplus_mma_enabled() && left >= 8) {
-            // subdomains too large for the vectors in shared memory: 16 (or 8) columns with the
-            // vectors in a global scratch instead of 2-4 columns per pass
-            const int ncg = left >= 16 ? 16 : 8;
-            const size_t need = (size_t)ncg * ((size_t)TILE * kp_tsum + (size_t)KPM_PAD * P.nd);
+        const bool s8 = smem(8) <= KP_SMEM_MAX, s16 = smem(16) <= KP_SMEM_MAX;
+        const int nc = left > 8 && (s16 || !s8) ? 16 : 8, nact = std::min(left, nc);
+        const bool gl = nc == 16 ? !s16 : !s8;
+        if (gl) {
+            const size_t need = (size_t)nc * ((size_t)TILE * kp_tsum + (size_t)KPM_PAD * P.nd);
             if (kp_gvec_n < need) {
                 kp_gvec = alloc<double>(need);
                 kp_gvec_n = need;
             }
-            if (ncg == 16) kplus_mma_kernel<16, true><<<P.nd, 256, 0, stream>>>(KP, in, out, mode, j0, ntot, z, kp_gvec);
-            else kplus_mma_kernel<8, true><<<P.nd, 256, 0, stream>>>(KP, in, out, mode, j0, ntot, z, kp_gvec);
-            CUDA_CHECK(cudaGetLastError());
-            j0 += ncg;
-            continue;
         }
-        switch (nc) {
-        case 16: kplus_multi_kernel<16><<<P.nd, 256, sm, stream>>>(KP, in, out, mode, j0, ntot, z); break;
-        case 8: kplus_multi_kernel<8><<<P.nd, 256, sm, stream>>>(KP, in, out, mode, j0, ntot, z); break;
-        case 4: kplus_multi_kernel<4><<<P.nd, 256, sm, stream>>>(KP, in, out, mode, j0, ntot, z); break;
-        case 2: kplus_multi_kernel<2><<<P.nd, 256, sm, stream>>>(KP, in, out, mode, j0, ntot, z); break;
-        default: kplus_multi_kernel<1><<<P.nd, 256, sm, stream>>>(KP, in, out, mode, j0, ntot, z); break;
-        }
-        CUDA_CHECK(cudaGetLastError());
-        j0 += nc;
+        auto kernel = nc == 16 ? (gl ? kplus_mma_kernel<16, true> : kplus_mma_kernel<16, false>)
+                               : (gl ? kplus_mma_kernel<8, true> : kplus_mma_kernel<8, false>);
+        launch_cluster(kernel, kp_cluster, dim3(P.nd * kp_cluster), dim3(KP_WARPS * 32), gl ? 0 : smem(nc), stream, KP, in,
+                       out, mode, j0, nact, ntot, z, kp_gvec);
+        j0 += nact;
     }
 }
 
@@ -2489,15 +2355,8 @@ void GpuSolver::Impl::upload_kplus(const Decomposition &dec, const Prep &prep, c
     CUDA_CHECK(cudaFuncSetAttribute(kplus_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)KP_SMEM_MAX));
     CUDA_CHECK(cudaFuncSetAttribute(kplus_dual_kernel<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)KP_SMEM_MAX));
     CUDA_CHECK(cudaFuncSetAttribute(kplus_dual_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)KP_SMEM_MAX));
-    CUDA_CHECK(cudaFuncSetAttribute(kplus_multi_kernel<16>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kplus_multi_smem(16)));
-    CUDA_CHECK(cudaFuncSetAttribute(kplus_multi_kernel<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kplus_multi_smem(8)));
-    CUDA_CHECK(cudaFuncSetAttribute(kplus_multi_kernel<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kplus_multi_smem(4)));
-    CUDA_CHECK(cudaFuncSetAttribute(kplus_multi_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kplus_multi_smem(2)));
-    CUDA_CHECK(cudaFuncSetAttribute(kplus_multi_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kplus_multi_smem(1)));
-    CUDA_CHECK(cudaFuncSetAttribute(kplus_mma_kernel<16, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    (int)kplus_mma_smem(16)));
-    CUDA_CHECK(cudaFuncSetAttribute(kplus_mma_kernel<8, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    (int)kplus_mma_smem(8)));
+    CUDA_CHECK(cudaFuncSetAttribute(kplus_mma_kernel<16, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)KP_SMEM_MAX));
+    CUDA_CHECK(cudaFuncSetAttribute(kplus_mma_kernel<8, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)KP_SMEM_MAX));
 }
 
 void GpuSolver::Impl::upload_hybrid(const Decomposition &dec, const Prep &prep) {

@@ -41,3 +41,22 @@ def test_kplus_and_solve(name):
     finally:
         inst.destroy()
         host.destroy()
+
+
+@pytest.mark.parametrize("name", ["heat_4", "elast_48", "elast_94", "uneven"])
+@pytest.mark.parametrize("nrhs", [2, 9, 17])
+def test_kplus_columns(name, nrhs):
+    """The multi-column K+ (padded groups of 8 and 16, a last single column; 94 blocks keep 8 columns in
+    shared memory) through whole solves: every column equals its own solve.  Both stop at 1e-11."""
+    P = CASES[name]()
+    inst = problems.make_instance(P, iopts={F.PRECONDITIONER: F.PREC_LUMPED, F.VERBOSE_LEVEL: 0, F.MAX_ITERATIONS: 2000},
+                                  ropts={F.PRECISION: 1e-11})
+    try:
+        R = problems.traction_loads(P, nrhs, seed=nrhs)
+        U = inst.solve_multi(R)
+        for j in (0, nrhs // 2, nrhs - 1):
+            inst.update_rhs(R[j])
+            u = inst.solve()
+            assert np.linalg.norm(U[j] - u) <= 1e-8 * np.linalg.norm(u)
+    finally:
+        inst.destroy()
