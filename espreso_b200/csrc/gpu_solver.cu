@@ -126,6 +126,8 @@ struct HybDev {
     const int *zof;               // nd+1: offsets of the subdomains' slots (m_i = zof[i+1] - zof[i])
     const int *m0;                // nd: B0 entries of the subdomain (first m0 columns of V_i)
     const int *vmap;              // per slot: index into its cluster's vector
+    const int *zsrc_ptr, *zsrc;   // per cluster vector entry (offset cof[c]): the slots that add into it, in
+                                  // member order
     const int *sub_cl;            // nd: cluster of every subdomain
     const int *cof;               // ncl+1: offsets of the cluster vectors
     const long long *mof;         // ncl: offset of M_c (nc x nc)
@@ -1773,35 +1775,49 @@ __device__ __forceinline__ bool hyb_skip(const DevProblem &P, int slot, int cond
     return cond == 3 && P.st->replace_iter != iter;
 }
 
-// z_i = V_i^T x_i: one warp per column of V_i.  With x == null the PCG direction
-// p = y + beta p is formed on the fly, as the tile SYMV does (update_kernel stores it later).
-__global__ void hyb_vt_kernel(DevProblem P, HybDev H, const double *x, int slot, int cond) {
+// z_i = V_i^T x_i, grid (nd, column groups): x_i is staged in shared memory, a warp takes a column at a
+// time with four loads in flight.  One CTA per subdomain left 64 subdomains on 64 SMs and formed the
+// direction again for every column.  The three kernels of the correction took 179 us per apply on 64
+// subdomains of 6^3 elasticity elements (81 + 45 + 52, cold caches); with the grids of this and the
+// next two kernels the solve went from 14.7 to 9.7 ms.  With x == null the PCG direction p = y + beta p is formed
+// on the fly, as the tile SYMV does (update_kernel stores it later).
+constexpr int HV_COLS = 16;
+__global__ void __launch_bounds__(256) hyb_vt_kernel(DevProblem P, HybDev H, const double *x, int slot, int cond) {
     pdl_enter();
     if (hyb_skip(P, slot, cond)) return;
+    extern __shared__ double hx[];
     const int d = blockIdx.x, lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
-    const int e0 = P.loff[d], ni = P.loff[d + 1] - e0;
     const int z0 = H.zof[d], m = H.zof[d + 1] - z0;
+    const int c0 = blockIdx.y * HV_COLS, c1 = min(m, c0 + HV_COLS);
+    if (c0 >= m) return;
+    const int e0 = P.loff[d], ni = P.loff[d + 1] - e0;
     const double *V = H.V + H.voff[d];
-    double beta = 0.0;
     if (x == nullptr) {
         const int iter = P.st->iter_base + slot;
-        beta = iter == 0 ? 0.0 : P.scal[SC_RHO] / P.rho_hist[iter - 1];
+        const double beta = iter == 0 ? 0.0 : P.scal[SC_RHO] / P.rho_hist[iter - 1];
+        for (int r = threadIdx.x; r < ni; r += blockDim.x) hx[r] = __ldg(P.y + e0 + r) + beta * __ldg(P.p + e0 + r);
+    } else {
+        for (int r = threadIdx.x; r < ni; r += blockDim.x) hx[r] = __ldg(x + e0 + r);
     }
-    for (int c = wid; c < m; c += nw) {
+    __syncthreads();
+    for (int c = c0 + wid; c < c1; c += nw) {
         const double *col = V + (size_t)c * ni;
-        double s = 0.0;
-        if (x == nullptr)
-            for (int r = lane; r < ni; r += 32) s += col[r] * (P.y[e0 + r] + beta * P.p[e0 + r]);
-        else
-            for (int r = lane; r < ni; r += 32) s += col[r] * x[e0 + r];
-        s = warp_sum(s);
-        if (lane == 0) H.z[z0 + c] = s;
+        double s[4] = {0.0, 0.0, 0.0, 0.0};
+        int r = lane;
+        for (; r + 96 < ni; r += 128)
+#pragma unroll
+            for (int k = 0; k < 4; ++k) s[k] += __ldg(col + r + 32 * k) * hx[r + 32 * k];
+        for (; r < ni; r += 32) s[0] += __ldg(col + r) * hx[r];
+        const double t = warp_sum((s[0] + s[1]) + (s[2] + s[3]));
+        if (lane == 0) H.z[z0 + c] = t;
     }
 }
 
 // w_c = M_c z_c for every cluster; z_c is gathered from the member slots in member order.
-// grid (ncl, row blocks); with dot != null the last CTA subtracts sum_c z_c . w_c from *dot.
-constexpr int HM_ROWS = 64;
+// grid (ncl, row blocks), two rows per warp; with dot != null the last CTA subtracts sum_c z_c . w_c from
+// *dot.  (Before: a pass over the members with a barrier each, and eight rows per warp.)
+constexpr int HM_ROWS = 64;    // rows per CTA of the block (multi right-hand-side) kernel
+constexpr int HM1_ROWS = 16;   // rows per CTA here
 __global__ void __launch_bounds__(256) hyb_m_kernel(DevProblem P, HybDev H, int slot, int cond, double *dot) {
     pdl_enter();
     if (hyb_skip(P, slot, cond)) return;
@@ -1809,27 +1825,31 @@ __global__ void __launch_bounds__(256) hyb_m_kernel(DevProblem P, HybDev H, int 
     __shared__ double sh[32];
     __shared__ int s_last;
     const int c = blockIdx.x;
-    const int nc = H.cof[c + 1] - H.cof[c];
-    for (int i = threadIdx.x; i < nc; i += blockDim.x) hz[i] = 0.0;
-    __syncthreads();
-    for (int q = H.mem_ptr[c]; q < H.mem_ptr[c + 1]; ++q) {
-        const int d = H.mem[q];
-        // the slots of one subdomain map to distinct entries of the cluster vector
-        for (int j = H.zof[d] + threadIdx.x; j < H.zof[d + 1]; j += blockDim.x) hz[H.vmap[j]] += H.z[j];
-        __syncthreads();
-    }
+    const int o = H.cof[c], nc = H.cof[c + 1] - o;
+    const int r0 = blockIdx.y * HM1_ROWS, r1 = min(nc, r0 + HM1_ROWS);
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
-    const int r0 = blockIdx.y * HM_ROWS, r1 = min(nc, r0 + HM_ROWS);
-    const double *M = H.M + H.mof[c];
     double zw = 0.0;
-    for (int r = r0 + wid; r < r1; r += nw) {
-        const double *col = M + (size_t)r * nc;    // symmetric: column r = row r
-        double s = 0.0;
-        for (int j = lane; j < nc; j += 32) s += col[j] * hz[j];
-        s = warp_sum(s);
-        if (lane == 0) {
-            H.w[H.cof[c] + r] = s;
-            zw += s * hz[r];
+    if (r0 < nc) {
+        for (int i = threadIdx.x; i < nc; i += blockDim.x) {
+            double s = 0.0;
+            for (int q = __ldg(H.zsrc_ptr + o + i); q < __ldg(H.zsrc_ptr + o + i + 1); ++q) s += __ldg(H.z + __ldg(H.zsrc + q));
+            hz[i] = s;
+        }
+        __syncthreads();
+        const double *M = H.M + H.mof[c];
+        for (int r = r0 + wid; r < r1; r += nw) {
+            const double *col = M + (size_t)r * nc;    // symmetric: column r = row r
+            double s[4] = {0.0, 0.0, 0.0, 0.0};
+            int j = lane;
+            for (; j + 96 < nc; j += 128)
+#pragma unroll
+                for (int k = 0; k < 4; ++k) s[k] += __ldg(col + j + 32 * k) * hz[j + 32 * k];
+            for (; j < nc; j += 32) s[0] += __ldg(col + j) * hz[j];
+            const double t = warp_sum((s[0] + s[1]) + (s[2] + s[3]));
+            if (lane == 0) {
+                H.w[o + r] = t;
+                zw += t * hz[r];
+            }
         }
     }
     if (dot == nullptr) return;
@@ -1853,23 +1873,34 @@ __global__ void __launch_bounds__(256) hyb_m_kernel(DevProblem P, HybDev H, int 
     }
 }
 
-// y_i -= V_i w_{c(i)}: one thread per row
-__global__ void hyb_v_kernel(DevProblem P, HybDev H, double *y, int slot, int cond) {
+// y_i -= V_i w_{c(i)}, grid (nd, row groups): a CTA takes HVR rows, its four quarters every fourth column
+// each, four loads in flight per thread.  (Before: one thread per row over all columns.)
+constexpr int HVR = 64;
+__global__ void __launch_bounds__(4 * HVR) hyb_v_kernel(DevProblem P, HybDev H, double *y, int slot, int cond) {
     pdl_enter();
     if (hyb_skip(P, slot, cond)) return;
     extern __shared__ double wl[];
+    __shared__ double part[4][HVR];
     const int d = blockIdx.x;
     const int e0 = P.loff[d], ni = P.loff[d + 1] - e0;
+    const int rr = threadIdx.x % HVR, g = threadIdx.x / HVR, r = blockIdx.y * HVR + rr;
+    if ((int)blockIdx.y * HVR >= ni) return;
     const int z0 = H.zof[d], m = H.zof[d + 1] - z0;
     const double *wc = H.w + H.cof[H.sub_cl[d]];
-    for (int j = threadIdx.x; j < m; j += blockDim.x) wl[j] = wc[H.vmap[z0 + j]];
+    for (int j = threadIdx.x; j < m; j += blockDim.x) wl[j] = __ldg(wc + __ldg(H.vmap + z0 + j));
     __syncthreads();
-    const double *V = H.V + H.voff[d];
-    for (int r = threadIdx.x; r < ni; r += blockDim.x) {
-        double s = 0.0;
-        for (int c = 0; c < m; ++c) s += V[(size_t)c * ni + r] * wl[c];
-        y[e0 + r] -= s;
+    double s[4] = {0.0, 0.0, 0.0, 0.0};
+    if (r < ni) {
+        const double *V = H.V + H.voff[d] + r;
+        int c = g;
+        for (; c + 12 < m; c += 16)
+#pragma unroll
+            for (int k = 0; k < 4; ++k) s[k] += __ldg(V + (size_t)(c + 4 * k) * ni) * wl[c + 4 * k];
+        for (; c < m; c += 4) s[0] += __ldg(V + (size_t)c * ni) * wl[c];
     }
+    part[g][rr] = (s[0] + s[1]) + (s[2] + s[3]);
+    __syncthreads();
+    if (g == 0 && r < ni) y[e0 + r] -= (part[0][rr] + part[1][rr]) + (part[2][rr] + part[3][rr]);
 }
 
 // cluster K^+ on primal vectors, step 1: z_i = [B0_i (K_i^+ x_i); -R_i^T x_i]
@@ -1997,7 +2028,7 @@ struct GpuSolver::Impl {
     // Hybrid Total FETI
     bool hybrid = false;
     HybDev H{};
-    int hyb_max_m = 0, hyb_rows = 1;
+    int hyb_max_m = 0, hyb_rows = 1, hyb_rows1 = 1;
     double *d_h = nullptr;              // primal scratch of the cluster K^+
     void upload_hybrid(const Decomposition &dec, const Prep &prep);
     // y -= V M V^T x (cond as hyb_skip; x null: the PCG direction y + beta p; dot: p.Ap to correct)
@@ -2416,6 +2447,18 @@ void GpuSolver::Impl::upload_hybrid(const Decomposition &dec, const Prep &prep) 
     H.zof = upload(zof);
     H.m0 = upload(m0);
     H.vmap = upload(vmap);
+    {
+        // the slots that add into every cluster vector entry, in member order
+        std::vector<int> ptr(cof[ncl] + 1, 0), src(zof[nd]);
+        for (int d = 0; d < nd; ++d)
+            for (int j = zof[d]; j < zof[d + 1]; ++j) ++ptr[cof[sub_cl[d]] + vmap[j] + 1];
+        for (int i = 0; i < cof[ncl]; ++i) ptr[i + 1] += ptr[i];
+        std::vector<int> at(ptr.begin(), ptr.end() - 1);
+        for (int d : mem)
+            for (int j = zof[d]; j < zof[d + 1]; ++j) src[at[cof[sub_cl[d]] + vmap[j]]++] = j;
+        H.zsrc_ptr = upload(ptr);
+        H.zsrc = upload(src);
+    }
     H.sub_cl = upload(sub_cl);
     H.cof = upload(cof);
     H.mof = upload(mof);
@@ -2429,19 +2472,23 @@ void GpuSolver::Impl::upload_hybrid(const Decomposition &dec, const Prep &prep) 
     H.w = alloc<double>(cof[ncl]);
     hyb_w_size = cof[ncl];
     hyb_rows = (max_nc + HM_ROWS - 1) / HM_ROWS;
-    H.part = alloc<double>((size_t)ncl * hyb_rows);
+    hyb_rows1 = (max_nc + HM1_ROWS - 1) / HM1_ROWS;
+    H.part = alloc<double>((size_t)ncl * hyb_rows1);
     H.done = alloc<int>(1);
     CUDA_CHECK(cudaMemset(H.done, 0, sizeof(int)));
     hyb_max_m = max_m;
+    CUDA_CHECK(cudaFuncSetAttribute(hyb_vt_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
     cudaFuncSetAttribute(hyb_m_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
     cudaFuncSetAttribute(hyb_v_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
 }
 
 void GpuSolver::Impl::launch_hybrid_F(const double *x, double *y, int slot, int cond, double *dot) {
     if (!hybrid) return;
-    launch_pdl(hyb_vt_kernel, dim3(P.nd), dim3(256), 0, stream, P, H, x, slot, cond);
-    launch_pdl(hyb_m_kernel, dim3(H.ncl, hyb_rows), dim3(256), sizeof(double) * H.max_nc, stream, P, H, slot, cond, dot);
-    launch_pdl(hyb_v_kernel, dim3(P.nd), dim3(256), sizeof(double) * hyb_max_m, stream, P, H, y, slot, cond);
+    launch_pdl(hyb_vt_kernel, dim3(P.nd, (hyb_max_m + HV_COLS - 1) / HV_COLS), dim3(256), sizeof(double) * max_ni, stream, P,
+               H, x, slot, cond);
+    launch_pdl(hyb_m_kernel, dim3(H.ncl, hyb_rows1), dim3(256), sizeof(double) * H.max_nc, stream, P, H, slot, cond, dot);
+    launch_pdl(hyb_v_kernel, dim3(P.nd, (max_ni + HVR - 1) / HVR), dim3(4 * HVR), sizeof(double) * hyb_max_m, stream, P, H, y,
+               slot, cond);
 }
 
 // K_c^+ (or K^+) on ncol columns (stride ntot): both K^+ passes of the cluster solve on all columns
@@ -2463,7 +2510,7 @@ void GpuSolver::Impl::launch_kplus_dual_multi(const double *in, double *out, int
         const double *inj = in + (size_t)j * ntot;
         double *outj = out + (size_t)j * ntot, *hj = hyb_hm + (size_t)j * ntot;
         hyb_kz_kernel<<<P.nd, 256, 0, stream>>>(P, H, d_doff, d_rofs, d_R, outj, inj);
-        hyb_m_kernel<<<dim3(H.ncl, hyb_rows), 256, sizeof(double) * H.max_nc, stream>>>(P, H, 0, 0, nullptr);
+        hyb_m_kernel<<<dim3(H.ncl, hyb_rows1), 256, sizeof(double) * H.max_nc, stream>>>(P, H, 0, 0, nullptr);
         hyb_copy_kernel<<<std::max(1, std::min(4096, (ntot + 255) / 256)), 256, 0, stream>>>(inj, hj, ntot);
         hyb_kb0_kernel<<<(P.nd + 127) / 128, 128, 0, stream>>>(P, H, d_doff, hj);
         CUDA_CHECK(cudaMemcpyAsync(hyb_wsave + (size_t)j * wn, H.w, sizeof(double) * wn, cudaMemcpyDeviceToDevice,
@@ -2482,7 +2529,7 @@ void GpuSolver::Impl::launch_kplus_dual(const double *in, double *out) {
     launch_kplus(in, out);
     if (!hybrid) return;
     hyb_kz_kernel<<<P.nd, 256, 0, stream>>>(P, H, d_doff, d_rofs, d_R, out, in);
-    hyb_m_kernel<<<dim3(H.ncl, hyb_rows), 256, sizeof(double) * H.max_nc, stream>>>(P, H, 0, 0, nullptr);
+    hyb_m_kernel<<<dim3(H.ncl, hyb_rows1), 256, sizeof(double) * H.max_nc, stream>>>(P, H, 0, 0, nullptr);
     hyb_copy_kernel<<<std::max(1, std::min(4096, (ntot + 255) / 256)), 256, 0, stream>>>(in, d_h, ntot);
     hyb_kb0_kernel<<<(P.nd + 127) / 128, 128, 0, stream>>>(P, H, d_doff, d_h);
     launch_kplus(d_h, out);
