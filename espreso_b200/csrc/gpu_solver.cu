@@ -39,6 +39,7 @@ namespace {
 constexpr int KMAX = 8;        // kernel dimension bound per subdomain (elasticity: 6)
 constexpr int TPB = 256;       // threads of the per-subdomain kernels
 constexpr int TPB1 = 512;      // threads of the single right-hand-side w/preconditioner kernel
+constexpr int ROW_TPB = 256;   // threads of the single right-hand-side kernels over all rows
 constexpr int TPBB = 1024;     // threads of the per-subdomain block (multi right-hand-side) kernels
 constexpr int TILE = 32;       // Schur tile edge
 constexpr unsigned FULL = 0xffffffffu;
@@ -333,44 +334,113 @@ __device__ void grid_total(double v, double *partials, int *counter, double *out
     }
 }
 
-// G_i v over the rows [e0, e1) of one subdomain, written to d[kof..]; KC = the row stride KS of the
-// coefficients (zero-padded rows), so only the problem's kernel width is reduced
-template <int KC>
-__device__ void g_dot_kc(const DevProblem &P, int dsub, const double *v, double *sh) {
-    const int e0 = P.loff[dsub], e1 = P.loff[dsub + 1];
-    const int nk = P.kof[dsub + 1] - P.kof[dsub];
-    double gk[KC];
-#pragma unroll
-    for (int k = 0; k < KC; ++k) gk[k] = 0.0;
-    for (int e = e0 + threadIdx.x; e < e1; e += blockDim.x) {
-        const double ve = v[e - e0];
-        const double *g = P.Gl + (size_t)e * KC;
-#pragma unroll
-        for (int k = 0; k < KC; ++k) gk[k] += __ldg(g + k) * ve;
-    }
-    block_sum_kc<KC>(gk, sh);
-    if (threadIdx.x == 0)
-        for (int k = 0; k < nk; ++k) P.d[P.kof[dsub] + k] = gk[k];
+__device__ __forceinline__ unsigned cluster_size_x() {
+    unsigned v;
+    asm volatile("mov.u32 %0, %%cluster_nctaid.x;" : "=r"(v));
+    return v;
+}
+__device__ __forceinline__ unsigned cluster_rank_x() {
+    unsigned v;
+    asm volatile("mov.u32 %0, %%cluster_ctaid.x;" : "=r"(v));
+    return v;
+}
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire;" ::: "memory"); }
+// the same shared-memory variable in CTA `rank` of the cluster
+__device__ __forceinline__ void st_cluster(double *p, unsigned rank, double v) {
+    unsigned a;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"((unsigned)__cvta_generic_to_shared(p)), "r"(rank));
+    asm volatile("st.shared::cluster.f64 [%0], %1;" ::"r"(a), "d"(v) : "memory");
 }
 
-__device__ void g_dot(const DevProblem &P, int dsub, const double *v, double *sh) {
-    if (P.KS == 1) { g_dot_kc<1>(P, dsub, v, sh); return; }
-    if (P.KS == 6) { g_dot_kc<6>(P, dsub, v, sh); return; }
-    const int e0 = P.loff[dsub], e1 = P.loff[dsub + 1];
-    const int nk = P.kof[dsub + 1] - P.kof[dsub];
-    double gk[KMAX];
+// Kernel widths: KC = the row stride KS of the coefficient arrays for the common problems (1 heat,
+// 6 elasticity, rows zero-padded), 0 for any other (per-row counts).
+template <int KC>
+constexpr int kwidth = KC ? KC : KMAX;
+
+// (G^T a) at local row e with the kernel width known at compile time
+template <int KC>
+__device__ __forceinline__ double gt_alpha_k(const DevProblem &P, int e, const double *a) {
+    if (KC == 6) {
+        // the six coefficients of a row as three 16-byte loads
+        const int ko = __ldg(P.rkof + e), po = __ldg(P.pkof + e);
+        const double2 *g = reinterpret_cast<const double2 *>(P.Gl + (size_t)e * 6);
+        const double2 *gp = reinterpret_cast<const double2 *>(P.Gp + (size_t)e * 6);
+        double s = 0.0;
 #pragma unroll
-    for (int k = 0; k < KMAX; ++k) gk[k] = 0.0;
-    for (int e = e0 + threadIdx.x; e < e1; e += blockDim.x) {
-        const double ve = v[e - e0];
-        const double *g = P.Gl + (size_t)e * P.KS;
+        for (int k = 0; k < 3; ++k) {
+            const double2 u = __ldg(g + k), w = __ldg(gp + k);
+            s += u.x * a[ko + 2 * k] + w.x * a[po + 2 * k];
+            s += u.y * a[ko + 2 * k + 1] + w.y * a[po + 2 * k + 1];
+        }
+        return s;
+    }
+    return KC ? gt_alpha_fixed<kwidth<KC>>(P, e, a) : gt_alpha(P, e, a);
+}
+
+// g += G_i v for one row
+template <int KC>
+__device__ __forceinline__ void g_add(const DevProblem &P, int e, double v, double (&g)[kwidth<KC>]) {
+    if (KC == 6) {
+        const double2 *c = reinterpret_cast<const double2 *>(P.Gl + (size_t)e * 6);
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+            const double2 u = __ldg(c + k);
+            g[2 * k] += u.x * v;
+            g[2 * k + 1] += u.y * v;
+        }
+    } else if (KC) {
+#pragma unroll
+        for (int k = 0; k < kwidth<KC>; ++k) g[k] += __ldg(P.Gl + (size_t)e * KC + k) * v;
+    } else {
+        const int nk = P.rnk[e];
 #pragma unroll
         for (int k = 0; k < KMAX; ++k)
-            if (k < nk) gk[k] += g[k] * ve;
+            if (k < nk) g[k] += __ldg(P.Gl + (size_t)e * P.KS + k) * v;
     }
-    block_sum_k(gk, sh);
-    if (threadIdx.x == 0)
-        for (int k = 0; k < nk; ++k) P.d[P.kof[dsub] + k] = gk[k];
+}
+
+// A kernel that writes to the shared memory of its cluster's other CTAs calls cluster_enter first and
+// cluster_entered before the first such write: by then every CTA of the cluster runs.
+__device__ __forceinline__ void cluster_enter() {
+    if (cluster_size_x() > 1) cluster_arrive();
+}
+__device__ __forceinline__ void cluster_entered() {
+    if (cluster_size_x() > 1) cluster_wait();
+}
+
+// Sums the threads' g over the CTAs of the subdomain's cluster (rank order) into d[kof..].  Every thread
+// of the cluster calls it, after cluster_enter.
+template <int KC>
+__device__ void g_finish(const DevProblem &P, int dsub, double (&g)[kwidth<KC>]) {
+    constexpr int K = kwidth<KC>;
+    __shared__ double sh[32 * K];
+    __shared__ double cl[8 * K];
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
+    const unsigned C = cluster_size_x(), rank = cluster_rank_x();
+#pragma unroll
+    for (int k = 0; k < K; ++k) {
+        const double t = warp_sum(g[k]);
+        if (lane == 0) sh[wid * K + k] = t;
+    }
+    __syncthreads();
+    cluster_entered();
+    const int nk = P.kof[dsub + 1] - P.kof[dsub];
+    for (int k = wid; k < K; k += nw) {
+        const double t = warp_sum(lane < nw ? sh[lane * K + k] : 0.0);
+        if (lane == 0) {
+            if (C > 1) st_cluster(&cl[rank * K + k], 0, t);
+            else if (k < nk) P.d[P.kof[dsub] + k] = t;
+        }
+    }
+    if (C == 1) return;
+    cluster_arrive();
+    cluster_wait();
+    if (rank == 0 && threadIdx.x < nk) {
+        double t = 0.0;
+        for (unsigned r = 0; r < C; ++r) t += cl[r * K + threadIdx.x];
+        P.d[P.kof[dsub] + threadIdx.x] = t;
+    }
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -896,38 +966,44 @@ __global__ void zero2_kernel(double *a, double *b, int n) {
     if (i < n) { a[i] = 0.0; b[i] = 0.0; }
 }
 
-// r = b - assemble(Ax); d = G r per subdomain; ||b||^2 total (initial call).  One CTA per subdomain.
+// The vector kernels of the single right-hand-side PCG take their rows from a cluster of C CTAs per
+// subdomain (vec_cluster): one CTA per subdomain leaves most of the chip idle when there are fewer
+// subdomains than resident CTAs, and each of these kernels is a chain of a few dependent loads.
+// Solves, one CTA / clusters (vec_cluster): 64 subdomains of 8^3 elasticity elements 5.71 / 5.13 ms, 64
+// uneven ones 13.6 / 12.7 ms, 27 with the Dirichlet preconditioner 2.08 / 1.76 ms, hybrid 9.7 / 8.6 ms.
+
+// r = b - assemble(Ax); d = G r per subdomain; ||b||^2 total (initial call).
+template <int KC>
 __global__ void __launch_bounds__(1024) r0_kernel(DevProblem P, double *Ax, int replace_mode, int slot) {
     pdl_enter();
-    extern __shared__ double rv_s[];
-    __shared__ double sh[32 * KMAX];
+    __shared__ double sh[32];
     if (replace_mode) {
         const int iter = P.st->iter_base + slot;
         if (skip_iter(P.st, iter) || P.st->replace_iter != iter) return;
     }
-    const int dsub = blockIdx.x;
+    cluster_enter();
+    const int C = (int)cluster_size_x(), dsub = blockIdx.x / C;
     const int e0 = P.loff[dsub], e1 = P.loff[dsub + 1];
-    double bb = 0.0;
-    for (int e = e0 + threadIdx.x; e < e1; e += blockDim.x) {
+    double bb = 0.0, g[kwidth<KC>] = {};
+    for (int e = e0 + cluster_rank_x() * blockDim.x + threadIdx.x; e < e1; e += C * blockDim.x) {
         const int q = P.partner[e];
         const double a = Ax[e] + (q >= 0 ? Ax[q] : 0.0);
         const double rv = P.bL[e] - a;
         P.r[e] = rv;
-        rv_s[e - e0] = rv;
+        g_add<KC>(P, e, rv, g);
         bb += P.bL[e] * P.bL[e] * P.minv[e];
     }
-    __syncthreads();
-    g_dot(P, dsub, rv_s, sh);
+    g_finish<KC>(P, dsub, g);
     if (!replace_mode) grid_total(block_sum(bb, sh), P.part_b, P.done + DONE_B, P.scal + SC_BN2, sh);
 }
 
 // ||P r||^2 with alpha = (GG^T)^-1 G r (initial stop tolerance)
+template <int KC>
 __global__ void pnorm_kernel(DevProblem P) {
     __shared__ double sh[32];
-    const int dsub = blockIdx.x;
     double s = 0.0;
-    for (int e = P.loff[dsub] + threadIdx.x; e < P.loff[dsub + 1]; e += blockDim.x) {
-        double u = P.r[e] - gt_alpha(P, e, P.alpha);
+    for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < P.NL; e += gridDim.x * blockDim.x) {
+        double u = P.r[e] - gt_alpha_k<KC>(P, e, P.alpha);
         s += u * u * P.minv[e];
     }
     grid_total(block_sum(s, sh), P.part_w, P.done + DONE_PN, P.scal + SC_PN2, sh);
@@ -941,103 +1017,129 @@ __global__ void tol_kernel(DevProblem P) {
     }
 }
 
-// w = r - G^T alpha (||w||^2 total), u_T = B^T (W w) and, for the lumped
-// preconditioner, v_T = K_TT u_T (sliced ELL).  With no preconditioner y = w
-// and rho = y.w is taken here.  One CTA per subdomain.
-template <int PRECOND>
-__global__ void __launch_bounds__(TPB1) w_prec_kernel(DevProblem P, int slot) {
+// w = r - G^T alpha (||w||^2 total), u_T = B^T (W w) and, for the lumped preconditioner, v_T = K_TT u_T
+// (sliced ELL).  With no preconditioner y = w and rho = y.w is taken here.  One cluster per subdomain:
+// its CTAs share the rows, then the touched DOFs (slice sl belongs to rank sl mod C), and exchange w and
+// u_T through distributed shared memory.  A slice's entries are dealt to `parts` warps, eight loads in
+// flight each: one warp over a row of up to 81 entries was the longest chain of the kernel.
+constexpr int ELL_PARTS = 4;
+template <int PRECOND, int KC>
+__global__ void __launch_bounds__(TPB1) w_prec_kernel(DevProblem P, int slot, int parts) {
     pdl_enter();
     extern __shared__ double sm[];
     __shared__ double sh[32];
     const int iter = P.st->iter_base + slot;
     if (skip_iter(P.st, iter)) return;
-    const int dsub = blockIdx.x;
-    const int e0 = P.loff[dsub], e1 = P.loff[dsub + 1];
-    const int t0 = P.toff[dsub], t1 = P.toff[dsub + 1], nt = t1 - t0;
-    double *wsm = sm;              // w of the subdomain rows
-    double *u = sm + (e1 - e0);    // B^T W w on the touched DOFs
+    cluster_enter();
+    const int C = (int)cluster_size_x(), rank = (int)cluster_rank_x(), dsub = blockIdx.x / C;
+    const int e0 = P.loff[dsub], ni = P.loff[dsub + 1] - e0;
+    const int t0 = P.toff[dsub], nt = P.toff[dsub + 1] - t0;
+    double *wsm = sm;          // w of the subdomain rows
+    double *u = sm + ni;       // B^T W w on the touched DOFs
+    double *acc = u + nt;      // parts x (32 x slices of this rank)
     double ww = 0.0;
-    for (int e = e0 + threadIdx.x; e < e1; e += blockDim.x) {
-        const double wv = __ldg(P.r + e) - gt_alpha(P, e, P.alpha);
+    cluster_entered();
+    for (int i = rank * blockDim.x + threadIdx.x; i < ni; i += C * blockDim.x) {
+        const int e = e0 + i;
+        const double wv = __ldg(P.r + e) - gt_alpha_k<KC>(P, e, P.alpha);
         P.w[e] = wv;
-        wsm[e - e0] = wv;
         if (PRECOND == PREC_NONE) P.y[e] = wv;
+        else if (C == 1) wsm[i] = wv;
+        else
+            for (int q = 0; q < C; ++q) st_cluster(wsm + i, (unsigned)q, wv);
         ww += wv * wv * __ldg(P.minv + e);
     }
-    ww = block_sum(ww, sh);  // also a barrier for wsm
+    if (PRECOND != PREC_NONE) {
+        cluster_arrive();
+        cluster_wait();
+        const int nsl = (nt + 31) / 32, mine = nsl > rank ? (nsl - rank + C - 1) / C : 0;
+        for (int q = threadIdx.x; q < 32 * mine; q += blockDim.x) {
+            const int t = 32 * (rank + (q >> 5) * C) + (q & 31);
+            if (t >= nt) continue;
+            double s = 0.0;
+            for (int j = __ldg(P.trow_ptr + t0 + t); j < __ldg(P.trow_ptr + t0 + t + 1); ++j) {
+                const int e = __ldg(P.trow_idx + j);
+                s += __ldg(P.ws + e) * wsm[e - e0];
+            }
+            if (PRECOND != PREC_LUMPED) P.uT[t0 + t] = s;
+            else if (C == 1) u[t] = s;
+            else
+                for (int r = 0; r < C; ++r) st_cluster(u + t, (unsigned)r, s);
+            if (PRECOND == PREC_WEIGHT) P.vT[t0 + t] = s;
+        }
+        if (PRECOND == PREC_LUMPED) {
+            cluster_arrive();
+            cluster_wait();
+            const int lane = threadIdx.x & 31, nw = blockDim.x >> 5, sl0 = P.slice0[dsub];
+            for (int q = threadIdx.x >> 5; q < mine * parts; q += nw) {
+                const int k = q / parts, pt = q - k * parts, sl = sl0 + rank + k * C;
+                const int wd = __ldg(P.ell_w + sl);
+                const int j0 = wd * pt / parts, j1 = wd * (pt + 1) / parts;
+                const int base = __ldg(P.ell_ptr + sl) + lane;
+                double s0 = 0.0, s1 = 0.0;
+                int j = j0;
+                for (; j + 8 <= j1; j += 8) {
+                    double v[8];
+                    int c[8];
+#pragma unroll
+                    for (int x = 0; x < 8; ++x) {
+                        v[x] = __ldg(P.ell_val + base + (j + x) * 32);
+                        c[x] = __ldg(P.ell_col + base + (j + x) * 32);
+                    }
+#pragma unroll
+                    for (int x = 0; x < 8; x += 2) {
+                        s0 += v[x] * u[c[x]];
+                        s1 += v[x + 1] * u[c[x + 1]];
+                    }
+                }
+#pragma unroll 4
+                for (; j < j1; ++j) s0 += __ldg(P.ell_val + base + j * 32) * u[__ldg(P.ell_col + base + j * 32)];
+                acc[(pt * mine + k) * 32 + lane] = s0 + s1;
+            }
+            __syncthreads();
+            for (int q = threadIdx.x; q < 32 * mine; q += blockDim.x) {
+                const int t = 32 * (rank + (q >> 5) * C) + (q & 31);
+                double s = 0.0;
+                for (int pt = 0; pt < parts; ++pt) s += acc[pt * mine * 32 + q];
+                if (t < nt) P.vT[t0 + t] = s;
+            }
+        }
+    }
+    ww = block_sum(ww, sh);
     grid_total(ww, P.part_w, P.done + DONE_W, P.scal + SC_WN2, sh);
-    if (PRECOND == PREC_NONE) {
-        grid_total(ww, P.part_rho, P.done + DONE_RHO, P.scal + SC_RHO, sh);
-        return;
-    }
-    for (int t = threadIdx.x; t < nt; t += blockDim.x) {
-        double s = 0.0;
-        for (int j = __ldg(P.trow_ptr + t0 + t); j < __ldg(P.trow_ptr + t0 + t + 1); ++j) {
-            const int e = __ldg(P.trow_idx + j);
-            s += __ldg(P.ws + e) * wsm[e - e0];
-        }
-        if (PRECOND == PREC_LUMPED) u[t] = s;
-        else P.uT[t0 + t] = s;
-        if (PRECOND == PREC_WEIGHT) P.vT[t0 + t] = s;
-    }
-    if (PRECOND != PREC_LUMPED) return;
-    __syncthreads();
-    const int sl0 = P.slice0[dsub];
-    for (int t = threadIdx.x; t < nt; t += blockDim.x) {
-        const int sl = sl0 + (t >> 5), ln = t & 31;
-        const int base = __ldg(P.ell_ptr + sl), wd = __ldg(P.ell_w + sl);
-        // four independent entries per step: their loads are in flight together
-        double s0 = 0.0, s1 = 0.0, s2 = 0.0, s3 = 0.0;
-        int j = 0;
-        for (; j + 3 < wd; j += 4) {
-            const int o = base + j * 32 + ln;
-            const double v0 = __ldg(P.ell_val + o), v1 = __ldg(P.ell_val + o + 32), v2 = __ldg(P.ell_val + o + 64),
-                         v3 = __ldg(P.ell_val + o + 96);
-            const int c0 = __ldg(P.ell_col + o), c1 = __ldg(P.ell_col + o + 32), c2 = __ldg(P.ell_col + o + 64),
-                      c3 = __ldg(P.ell_col + o + 96);
-            s0 += v0 * u[c0];
-            s1 += v1 * u[c1];
-            s2 += v2 * u[c2];
-            s3 += v3 * u[c3];
-        }
-        for (; j < wd; ++j) {
-            const int o = base + j * 32 + ln;
-            s0 += __ldg(P.ell_val + o) * u[__ldg(P.ell_col + o)];
-        }
-        P.vT[t0 + t] = (s0 + s1) + (s2 + s3);
-    }
+    if (PRECOND == PREC_NONE) grid_total(ww, P.part_rho, P.done + DONE_RHO, P.scal + SC_RHO, sh);
 }
 
-// z = assemble(W B v_T); d = G z.  One CTA per subdomain.
+// z = assemble(W B v_T); d = G z.
+template <int KC>
 __global__ void __launch_bounds__(1024) z_kernel(DevProblem P, int slot) {
     pdl_enter();
-    extern __shared__ double zs[];
-    __shared__ double sh[32 * KMAX];
     const int iter = P.st->iter_base + slot;
     if (skip_iter(P.st, iter)) return;
-    const int dsub = blockIdx.x;
+    cluster_enter();
+    const int C = (int)cluster_size_x(), dsub = blockIdx.x / C;
     const int e0 = P.loff[dsub], e1 = P.loff[dsub + 1];
-    for (int e = e0 + threadIdx.x; e < e1; e += blockDim.x) {
+    double g[kwidth<KC>] = {};
+    for (int e = e0 + cluster_rank_x() * blockDim.x + threadIdx.x; e < e1; e += C * blockDim.x) {
         const int pt = __ldg(P.ptidx + e);
         double zv = __ldg(P.ws + e) * __ldg(P.vT + __ldg(P.tidx + e));
         if (pt >= 0) zv += __ldg(P.pws + e) * __ldg(P.vT + pt);
         P.z[e] = zv;
-        zs[e - e0] = zv;
+        g_add<KC>(P, e, zv, g);
     }
-    __syncthreads();
-    g_dot(P, dsub, zs, sh);
+    g_finish<KC>(P, dsub, g);
 }
 
 // y = z - G^T alpha, rho = y.w total; clear the F apply accumulators.
-__global__ void __launch_bounds__(1024) y_kernel(DevProblem P, double *Ax64, int slot) {
+template <int KC>
+__global__ void __launch_bounds__(512) y_kernel(DevProblem P, double *Ax64, int slot) {
     pdl_enter();
     __shared__ double sh[32];
     const int iter = P.st->iter_base + slot;
     if (skip_iter(P.st, iter)) return;
-    const int dsub = blockIdx.x;
     double s = 0.0;
-    for (int e = P.loff[dsub] + threadIdx.x; e < P.loff[dsub + 1]; e += blockDim.x) {
-        const double yv = __ldg(P.z + e) - gt_alpha(P, e, P.alpha);
+    for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < P.NL; e += gridDim.x * blockDim.x) {
+        const double yv = __ldg(P.z + e) - gt_alpha_k<KC>(P, e, P.alpha);
         P.y[e] = yv;
         s += yv * __ldg(P.w + e) * __ldg(P.minv + e);
         P.Ap[e] = 0.0;
@@ -1061,10 +1163,9 @@ struct LoopCtl {
     cudaGraphConditionalHandle h_loop, h_repl;
 };
 
+template <int KC>
 __global__ void __launch_bounds__(1024) update_kernel(DevProblem P, int slot) {
     pdl_enter();
-    extern __shared__ double rs_s[];
-    __shared__ double sh[32 * KMAX];
     const int iter = P.st->iter_base + slot;
     if (skip_iter(P.st, iter)) return;
     const double rho = P.scal[SC_RHO];
@@ -1072,9 +1173,11 @@ __global__ void __launch_bounds__(1024) update_kernel(DevProblem P, int slot) {
     const double wn2 = P.scal[SC_WN2];
     const double beta = (iter == 0) ? 0.0 : rho / P.rho_hist[iter - 1];
     const double alpha = rho / pAp;
-    const int dsub = blockIdx.x;
+    cluster_enter();
+    const int C = (int)cluster_size_x(), dsub = blockIdx.x / C;
     const int e0 = P.loff[dsub], e1 = P.loff[dsub + 1];
-    for (int e = e0 + threadIdx.x; e < e1; e += blockDim.x) {
+    double g[kwidth<KC>] = {};
+    for (int e = e0 + cluster_rank_x() * blockDim.x + threadIdx.x; e < e1; e += C * blockDim.x) {
         const int q = __ldg(P.partner + e);
         const double ap = __ldg(P.Ap + e) + (q >= 0 ? __ldg(P.Ap + q) : 0.0);
         const double pv = __ldg(P.y + e) + beta * P.p[e];
@@ -1082,10 +1185,9 @@ __global__ void __launch_bounds__(1024) update_kernel(DevProblem P, int slot) {
         P.x[e] += alpha * pv;
         const double rv = P.r[e] - alpha * ap;
         P.r[e] = rv;
-        rs_s[e - e0] = rv;
+        g_add<KC>(P, e, rv, g);
     }
-    __syncthreads();
-    g_dot(P, dsub, rs_s, sh);
+    g_finish<KC>(P, dsub, g);
     if (blockIdx.x == 0 && threadIdx.x == 0) {
         DevState *st = P.st;
         P.rho_hist[iter] = rho;
@@ -1261,25 +1363,6 @@ __device__ __forceinline__ long long ltile(int T, int I, int J) {
 // of nonzero tiles) 905 / 255 us, 64 uneven ones of up to 7,560 DOFs (largest 0.14 GB) 5.2 / 1.5 ms, 27
 // of 6^3 271 / 100 us; 512 of 10^3 heat elements fill the chip either way (592 us, clusters of one).
 constexpr int KP_WARPS = 8;
-
-__device__ __forceinline__ unsigned cluster_size_x() {
-    unsigned v;
-    asm volatile("mov.u32 %0, %%cluster_nctaid.x;" : "=r"(v));
-    return v;
-}
-__device__ __forceinline__ unsigned cluster_rank_x() {
-    unsigned v;
-    asm volatile("mov.u32 %0, %%cluster_ctaid.x;" : "=r"(v));
-    return v;
-}
-__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release;" ::: "memory"); }
-__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire;" ::: "memory"); }
-// the same shared-memory variable in CTA `rank` of the cluster
-__device__ __forceinline__ void st_cluster(double *p, unsigned rank, double v) {
-    unsigned a;
-    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"((unsigned)__cvta_generic_to_shared(p)), "r"(rank));
-    asm volatile("st.shared::cluster.f64 [%0], %1;" ::"r"(a), "d"(v) : "memory");
-}
 
 struct KpTile {
     uint4 u[16];
@@ -1497,7 +1580,7 @@ __global__ void __launch_bounds__(KP_WARPS * 32, 2) kplus_dual_kernel(KplusDev K
             out[e] += yv;
         }
     }
-    if (MODE == 1) grid_total(block_sum(dot, sh), P.part_w + P.nd, P.done + DONE_PAP_IMPLICIT, P.scal + SC_PAP, sh);
+    if (MODE == 1) grid_total(block_sum(dot, sh), P.part_w + 8 * P.nd, P.done + DONE_PAP_IMPLICIT, P.scal + SC_PAP, sh);
 }
 
 // K^+ on NC = 8 or 16 right-hand sides (columns j0 .. j0+NC-1 of in/out, `stride` doubles apart; columns
@@ -2001,6 +2084,11 @@ struct GpuSolver::Impl {
     // threads of the per-subdomain vector kernels of the PCG loop: as many as keep every subdomain's
     // CTA resident in one wave (2048 threads per SM), so that each thread has about one row
     int tpbv = 256;
+    int vec_cluster = 1;      // CTAs per subdomain of the vector kernels
+    int ell_parts = 1;
+    size_t w_smem = 0;
+    int row_grid() const { return std::max(1, std::min(4 * nsm, (P.NL + ROW_TPB - 1) / ROW_TPB)); }
+    void launch_r0(int replace_mode, int slot);
     std::vector<int> h_lam;       // L row -> lambda
     int *d_lam = nullptr;         // the same on the device
     std::vector<int> h_loff;
@@ -2847,22 +2935,38 @@ static void set_smem_limits() {
     set_tile_limits<SCHUR_FP64>(v);
     set_tile_limits<SCHUR_FP32>(v);
     set_tile_limits<SCHUR_BF16>(v);
-    cudaFuncSetAttribute(w_prec_kernel<PREC_NONE>, cudaFuncAttributeMaxDynamicSharedMemorySize, v);
-    cudaFuncSetAttribute(w_prec_kernel<PREC_LUMPED>, cudaFuncAttributeMaxDynamicSharedMemorySize, v);
-    cudaFuncSetAttribute(w_prec_kernel<PREC_WEIGHT>, cudaFuncAttributeMaxDynamicSharedMemorySize, v);
-    cudaFuncSetAttribute(w_prec_kernel<PREC_DIRICHLET>, cudaFuncAttributeMaxDynamicSharedMemorySize, v);
-    cudaFuncSetAttribute(r0_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, v);
-    cudaFuncSetAttribute(z_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, v);
-    cudaFuncSetAttribute(update_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, v);
+    auto w_limits = [&](auto kc) {
+        constexpr int KC = decltype(kc)::value;
+        CUDA_CHECK(cudaFuncSetAttribute(w_prec_kernel<PREC_LUMPED, KC>, cudaFuncAttributeMaxDynamicSharedMemorySize, v));
+        CUDA_CHECK(cudaFuncSetAttribute(w_prec_kernel<PREC_WEIGHT, KC>, cudaFuncAttributeMaxDynamicSharedMemorySize, v));
+        CUDA_CHECK(cudaFuncSetAttribute(w_prec_kernel<PREC_DIRICHLET, KC>, cudaFuncAttributeMaxDynamicSharedMemorySize, v));
+    };
+    w_limits(std::integral_constant<int, 0>());
+    w_limits(std::integral_constant<int, 1>());
+    w_limits(std::integral_constant<int, 6>());
     done = true;
+}
+
+// f(integral constant) with the kernel width of the problem
+template <typename F>
+static void with_kwidth(int KS, F &&f) {
+    if (KS == 1) f(std::integral_constant<int, 1>());
+    else if (KS == 6) f(std::integral_constant<int, 6>());
+    else f(std::integral_constant<int, 0>());
+}
+
+void GpuSolver::Impl::launch_r0(int replace_mode, int slot) {
+    with_kwidth(P.KS, [&](auto kc) {
+        launch_cluster(r0_kernel<decltype(kc)::value>, vec_cluster, dim3(P.nd * vec_cluster), dim3(tpbv), 0, stream, P, Ax64,
+                       replace_mode, slot);
+    });
 }
 
 // One PCG iteration (reference order: w = P r, z = M w, y = P z, p, F p, update).
 void GpuSolver::Impl::launch_replacement(int slot) {
-    const int nd = P.nd;
     launch_tiles(F64, 3, P.x, nullptr, Ax64, slot);
     launch_hybrid_F(P.x, Ax64, slot, 3, nullptr);
-    launch_pdl(r0_kernel, dim3(nd), dim3(tpbv), sizeof(double) * max_ni, stream, P, Ax64, 1, slot);
+    launch_r0(1, slot);
 }
 
 void GpuSolver::Impl::launch_iteration(int slot, bool with_replacement, LoopCtl lc) {
@@ -2874,31 +2978,40 @@ void GpuSolver::Impl::launch_iteration(int slot, bool with_replacement, LoopCtl 
         // residual replacement r = b - F64 x when the previous update asked for it
         launch_tiles(F64, 3, P.x, nullptr, Ax64, slot);
         launch_hybrid_F(P.x, Ax64, slot, 3, nullptr);
-        launch_pdl(r0_kernel, dim3(nd), dim3(tpbv), sizeof(double) * max_ni, stream, P, Ax64, 1, slot);
+        launch_r0(1, slot);
     }
     launch_pdl(coarse_kernel, dim3(cgrid), dim3(256), 0, stream, P, P.d, P.alpha, slot, 1);
-    const size_t tsm = sizeof(double) * (size_t)(max_ni + max_nt);
-    switch (opt.precond) {
-    case PREC_NONE: launch_pdl(w_prec_kernel<PREC_NONE>, dim3(nd), dim3(TPB1), tsm, stream, P, slot); break;
-    case PREC_LUMPED: launch_pdl(w_prec_kernel<PREC_LUMPED>, dim3(nd), dim3(TPB1), tsm, stream, P, slot); break;
-    case PREC_WEIGHT: launch_pdl(w_prec_kernel<PREC_WEIGHT>, dim3(nd), dim3(TPB1), tsm, stream, P, slot); break;
-    default: launch_pdl(w_prec_kernel<PREC_DIRICHLET>, dim3(nd), dim3(TPB1), tsm, stream, P, slot); break;
-    }
+    const dim3 vgrid(P.nd * vec_cluster);
+    with_kwidth(P.KS, [&](auto kc) {
+        constexpr int KC = decltype(kc)::value;
+        auto w_prec = opt.precond == PREC_NONE     ? w_prec_kernel<PREC_NONE, KC>
+                      : opt.precond == PREC_LUMPED ? w_prec_kernel<PREC_LUMPED, KC>
+                      : opt.precond == PREC_WEIGHT ? w_prec_kernel<PREC_WEIGHT, KC>
+                                                   : w_prec_kernel<PREC_DIRICHLET, KC>;
+        launch_cluster(w_prec, vec_cluster, vgrid, dim3(vec_cluster > 1 ? TPB1 / 2 : TPB1),
+                       opt.precond == PREC_NONE ? 0 : w_smem, stream, P, slot, ell_parts);
+    });
     if (opt.precond != PREC_NONE) {
         if (opt.precond == PREC_DIRICHLET) {
             launch_pdl(zero_vT_kernel, dim3(std::max(1, std::min(1024, (P.NT + 255) / 256))), dim3(256), 0, stream, P,
                        slot);
             launch_tiles(Dir, 2, P.uT, nullptr, P.vT, slot);
         }
-        launch_pdl(z_kernel, dim3(nd), dim3(tpbv), sizeof(double) * max_ni, stream, P, slot);
+        with_kwidth(P.KS, [&](auto kc) {
+            launch_cluster(z_kernel<decltype(kc)::value>, vec_cluster, vgrid, dim3(tpbv), 0, stream, P, slot);
+        });
         launch_pdl(coarse_kernel, dim3(cgrid), dim3(256), 0, stream, P, P.d, P.alpha, slot, 1);
-        launch_pdl(y_kernel, dim3(nd), dim3(tpbv), 0, stream, P, Ax64, slot);
+        with_kwidth(P.KS, [&](auto kc) {
+            launch_pdl(y_kernel<decltype(kc)::value>, dim3(row_grid()), dim3(ROW_TPB), 0, stream, P, Ax64, slot);
+        });
     } else {
         launch_pdl(zero2_kernel, dim3((P.NL + 255) / 256), dim3(256), 0, stream, P.Ap, Ax64, P.NL);
     }
     launch_tiles(Fop, 1, P.y, P.p, P.Ap, slot);
     launch_hybrid_F(nullptr, P.Ap, slot, 1, P.scal + SC_PAP);   // p = y + beta p formed on the fly
-    launch_pdl(update_kernel, dim3(nd), dim3(tpbv), sizeof(double) * max_ni, stream, P, slot);
+    with_kwidth(P.KS, [&](auto kc) {
+        launch_cluster(update_kernel<decltype(kc)::value>, vec_cluster, vgrid, dim3(tpbv), 0, stream, P, slot);
+    });
     (void)lc;
 }
 
@@ -3048,8 +3161,16 @@ void GpuSolver::upload(const Decomposition &dec, const Prep &prep, const SolveOp
     I.n_lambda = dec.n_lambda;
     I.h_loff = loff;
     {
-        const int per_sm = std::max(1, (nd + I.nsm - 1) / I.nsm);
-        I.tpbv = std::max(128, std::min(1024, (2048 / per_sm) / 32 * 32));
+        // Clusters of the vector kernels: up to 8 CTAs per subdomain while all of them stay resident
+        // (four CTAs per SM) and each keeps 64 rows or more; then as many threads as have a row and
+        // fit the chip in one wave.
+        int max_rows = 1;
+        for (int d = 0; d < nd; ++d) max_rows = std::max(max_rows, prep.sub[d].ni);
+        I.vec_cluster = 1;
+        while (I.vec_cluster < 8 && 2 * I.vec_cluster * nd <= 4 * I.nsm && max_rows >= 128 * I.vec_cluster) I.vec_cluster *= 2;
+        const int per_sm = std::max(1, (nd * I.vec_cluster + I.nsm - 1) / I.nsm);
+        const int rows = ((max_rows + I.vec_cluster - 1) / I.vec_cluster + 31) / 32 * 32;
+        I.tpbv = std::max(128, std::min({1024, rows, (2048 / per_sm) / 32 * 32}));
     }
     I.h_lam.resize(NL);
     int KS = 1;
@@ -3131,6 +3252,13 @@ void GpuSolver::upload(const Decomposition &dec, const Prep &prep, const SolveOp
             tbase[t] = toff[d];
             tslot[t] = ((slice0[d] + ((t - toff[d]) >> 5)) << 5) | ((t - toff[d]) & 31);
         }
+    {
+        const int slices = ((I.max_nt + 31) / 32 + I.vec_cluster - 1) / I.vec_cluster;
+        auto bytes = [&](int parts) { return sizeof(double) * (size_t)(I.max_ni + I.max_nt + 32 * parts * slices); };
+        I.ell_parts = ELL_PARTS;
+        while (I.ell_parts > 1 && bytes(I.ell_parts) > 200 * 1024) I.ell_parts /= 2;
+        I.w_smem = bytes(I.ell_parts);
+    }
     FETI_CHECK(sizeof(double) * (size_t)(I.max_nt + I.max_ni) <= 200 * 1024,
                "FETI4I: subdomain interface too large for the preconditioner kernel");
 
@@ -3179,8 +3307,8 @@ void GpuSolver::upload(const Decomposition &dec, const Prep &prep, const SolveOp
     P.alpha = I.alloc<double>(prep.n_kern + KS);
     CUDA_CHECK(cudaMemset(P.alpha, 0, sizeof(double) * (prep.n_kern + KS)));
     I.e_dev = I.alloc<double>(P.nP);
-    P.part_w = I.alloc<double>(9 * (size_t)nd);   // the second part: up to 8 CTAs per subdomain (implicit F)
-    P.part_rho = I.alloc<double>(nd); P.part_b = I.alloc<double>(nd);
+    P.part_w = I.alloc<double>((size_t)16 * nd + I.row_grid());   // up to 8 CTAs per subdomain; second part: implicit F
+    P.part_rho = I.alloc<double>((size_t)8 * nd + I.row_grid()); P.part_b = I.alloc<double>((size_t)8 * nd);
     P.rho_hist = I.alloc<double>((size_t)opt.max_iterations + 64);
     I.st = I.alloc<DevState>(1);
     P.st = I.st;
@@ -3423,10 +3551,10 @@ void GpuSolver::solve(SolveStats &stats) {
     zero_kernel<<<(P.NL + 255) / 256, 256, 0, I.stream>>>(P.p, P.NL);
     I.launch_tiles(I.F64, 0, P.x, nullptr, I.Ax64, 0);
     I.launch_hybrid_F(P.x, I.Ax64, 0, 0, nullptr);
-    r0_kernel<<<nd, TPB, sizeof(double) * I.max_ni, I.stream>>>(P, I.Ax64, 0, 0);
+    I.launch_r0(0, 0);
     zero_kernel<<<(P.NL + 255) / 256, 256, 0, I.stream>>>(I.Ax64, P.NL);
     coarse_kernel<<<cgrid, 256, 0, I.stream>>>(P, P.d, P.alpha, 0, 0);
-    pnorm_kernel<<<nd, TPB, 0, I.stream>>>(P);
+    with_kwidth(P.KS, [&](auto kc) { pnorm_kernel<decltype(kc)::value><<<I.row_grid(), ROW_TPB, 0, I.stream>>>(P); });
     tol_kernel<<<1, 256, 0, I.stream>>>(P);
     CUDA_CHECK(cudaGetLastError());
     int launches = 9;
