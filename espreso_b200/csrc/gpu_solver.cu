@@ -166,17 +166,24 @@ struct TileSetDev {
 // off by default.
 __device__ __forceinline__ void pdl_enter() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
-// The dual PCG as one graph with conditional nodes (capture_loop), opt-in (FETI4I_LOOP_GRAPH=1).
-// It launches only the kernels an iteration needs (no replacement kernels that return at once, no
-// iterations past convergence in the last chunk): 258 instead of 300 launches per solve of the heat
-// workload of 216 subdomains, but measured 3.35 ms per solve against 3.28 ms with chunked graphs of
-// 16 iterations, so the chunked graphs stay the default.
-bool loop_graph_enabled() {
-    static const bool on = [] {
+// The dual PCG as one graph with a WHILE node (capture_loop).
+//   LOOP_BODY (default): the body is LOOP_STEP iterations, so a solve launches at most LOOP_STEP - 1
+//     iterations past convergence and waits for the host once.  Chunks of 16 iterations with a host
+//     check each ran up to 15 iterations of kernels that return at once (2-3 us each): 877 / 815 us per
+//     solve of 8 small heat subdomains (17 iterations), 1.76 / 1.65 ms of 27 with the Dirichlet
+//     preconditioner (18), 8.6 / 8.4 ms of the hybrid case (65); no difference at 30 of 32.
+//   LOOP_SINGLE (FETI4I_LOOP_GRAPH=1): one iteration per pass and an IF node for the residual
+//     replacement; fewest launches, but the conditional nodes of every pass cost more than they save
+//     (3.35 ms per solve of the heat workload of 216 subdomains against 3.28 ms with chunks of 16).
+//   LOOP_CHUNKS (FETI4I_LOOP_GRAPH=0, and where conditional nodes are refused): chunks of 16.
+enum LoopKind { LOOP_CHUNKS, LOOP_SINGLE, LOOP_BODY };
+constexpr int LOOP_STEP = 4;
+LoopKind loop_kind() {
+    static const LoopKind k = [] {
         const char *e = getenv("FETI4I_LOOP_GRAPH");
-        return e && e[0] == '1';
+        return e && e[0] == '1' ? LOOP_SINGLE : e && e[0] == '0' ? LOOP_CHUNKS : LOOP_BODY;
     }();
-    return on;
+    return k;
 }
 
 bool pdl_enabled() {
@@ -1159,7 +1166,8 @@ __global__ void zero_vT_kernel(DevProblem P, int slot) {
 // Device-side loop control (graph_loop): the WHILE node repeats the iteration while h_loop is
 // non-zero, the IF node at the top of an iteration runs the residual replacement when h_repl is.
 struct LoopCtl {
-    int on;                              // 0: launched outside the conditional graph
+    int step;                            // iterations per pass of the loop
+    int repl;                            // 1: h_repl is in use
     cudaGraphConditionalHandle h_loop, h_repl;
 };
 
@@ -1233,9 +1241,9 @@ __global__ void chunk_end_kernel(DevProblem P, int chunk) {
 __global__ void loop_end_kernel(DevProblem P, LoopCtl lc) {
     if (threadIdx.x == 0 && blockIdx.x == 0) {
         DevState *st = P.st;
-        const int done = ++st->iter_base;
+        const int done = st->iter_base += lc.step;
         const bool more = st->conv_iter < 0 && done < st->max_it && st->error == 0;
-        cudaGraphSetConditional(lc.h_repl, (more && st->replace_iter == done) ? 1u : 0u);
+        if (lc.repl) cudaGraphSetConditional(lc.h_repl, (more && st->replace_iter == done) ? 1u : 0u);
         cudaGraphSetConditional(lc.h_loop, more ? 1u : 0u);
     }
 }
@@ -2224,7 +2232,7 @@ struct GpuSolver::Impl {
     int graph_loop_key = -1;
     bool loop_refused = false;
     void launch_replacement(int slot);
-    void launch_iteration(int slot, bool with_replacement = true, LoopCtl lc = LoopCtl{0, 0, 0});
+    void launch_iteration(int slot, bool with_replacement = true);
     int kernels_per_iteration() const;
     void upload_kplus(const Decomposition &dec, const Prep &prep, const std::vector<int> &loff,
                       const std::vector<int> &toff);
@@ -2969,7 +2977,7 @@ void GpuSolver::Impl::launch_replacement(int slot) {
     launch_r0(1, slot);
 }
 
-void GpuSolver::Impl::launch_iteration(int slot, bool with_replacement, LoopCtl lc) {
+void GpuSolver::Impl::launch_iteration(int slot, bool with_replacement) {
     const int nd = P.nd;
     const int cgrid = (P.nK + 7) / 8;
     const bool mixed = opt.schur_precision != SCHUR_FP64;
@@ -3012,7 +3020,6 @@ void GpuSolver::Impl::launch_iteration(int slot, bool with_replacement, LoopCtl 
     with_kwidth(P.KS, [&](auto kc) {
         launch_cluster(update_kernel<decltype(kc)::value>, vec_cluster, vgrid, dim3(tpbv), 0, stream, P, slot);
     });
-    (void)lc;
 }
 
 int GpuSolver::Impl::kernels_per_iteration() const {
@@ -3041,19 +3048,20 @@ void GpuSolver::Impl::capture_chunk(int chunk) {
     graph_precond = opt.precond;
 }
 
-// The whole dual PCG as one graph: a WHILE node around one iteration (its slot 0, iter_base advanced
-// by one per pass) and, in mixed precision, an IF node at its top for the residual replacement.
-// update_kernel sets the IF condition and loop_end_kernel the WHILE condition, so the loop stops at
-// the converged iteration and no replacement kernels are launched in the iterations that do not
-// replace.  Returns false when the runtime refuses conditional nodes (graph chunks are used then).
+// The whole dual PCG as one graph: a WHILE node around LOOP_STEP iterations (slots 0 .. LOOP_STEP-1,
+// iter_base advanced per pass), or around one iteration with, in mixed precision, an IF node at its top
+// for the residual replacement (loop_kind).  loop_end_kernel sets the WHILE condition, so the loop stops
+// after the pass with the converged iteration.  Returns false when the runtime refuses conditional
+// nodes (graph chunks are used then).
 bool GpuSolver::Impl::capture_loop() {
     const int key = opt.schur_precision * 16 + opt.precond;
     if (graph_loop && graph_loop_key == key) return true;
     if (graph_loop) { cudaGraphExecDestroy(graph_loop); graph_loop = nullptr; }
-    if (pdl_enabled() || loop_refused || !loop_graph_enabled()) return false;
-    const bool mixed = opt.schur_precision != SCHUR_FP64;
+    const LoopKind kind = loop_kind();
+    if (pdl_enabled() || loop_refused || kind == LOOP_CHUNKS) return false;
+    const bool single = kind == LOOP_SINGLE, repl = single && opt.schur_precision != SCHUR_FP64;
     cudaGraph_t g = nullptr, tmp = nullptr;
-    LoopCtl lc{1, 0, 0};
+    LoopCtl lc{single ? 1 : LOOP_STEP, repl ? 1 : 0, 0, 0};
     auto fail = [&](cudaError_t e) {
         FETI_LOG(1, "FETI4I: conditional graph nodes unavailable (%s); using graph chunks\n", cudaGetErrorString(e));
         cudaStreamCaptureStatus cs;
@@ -3067,7 +3075,8 @@ bool GpuSolver::Impl::capture_loop() {
     cudaError_t e = cudaGraphCreate(&g, 0);
     if (e != cudaSuccess) return fail(e);
     if ((e = cudaGraphConditionalHandleCreate(&lc.h_loop, g, 1, cudaGraphCondAssignDefault)) != cudaSuccess) return fail(e);
-    if ((e = cudaGraphConditionalHandleCreate(&lc.h_repl, g, 0, cudaGraphCondAssignDefault)) != cudaSuccess) return fail(e);
+    if (repl && (e = cudaGraphConditionalHandleCreate(&lc.h_repl, g, 0, cudaGraphCondAssignDefault)) != cudaSuccess)
+        return fail(e);
     cudaGraphNodeParams wp = {};
     wp.type = cudaGraphNodeTypeConditional;
     wp.conditional.handle = lc.h_loop;
@@ -3077,7 +3086,7 @@ bool GpuSolver::Impl::capture_loop() {
     if ((e = cudaGraphAddNode(&wnode, g, nullptr, 0, &wp)) != cudaSuccess) return fail(e);
     cudaGraph_t body = wp.conditional.phGraph_out[0];
     cudaGraphNode_t top = nullptr;
-    if (mixed) {
+    if (repl) {
         cudaGraphNodeParams ip = {};
         ip.type = cudaGraphNodeTypeConditional;
         ip.conditional.handle = lc.h_repl;
@@ -3093,7 +3102,7 @@ bool GpuSolver::Impl::capture_loop() {
     if ((e = cudaStreamBeginCaptureToGraph(stream, body, top ? &top : nullptr, nullptr, top ? 1 : 0,
                                            cudaStreamCaptureModeThreadLocal)) != cudaSuccess)
         return fail(e);
-    launch_iteration(0, false, lc);
+    for (int j = 0; j < lc.step; ++j) launch_iteration(j, !single);
     loop_end_kernel<<<1, 32, 0, stream>>>(P, lc);
     if ((e = cudaStreamEndCapture(stream, &tmp)) != cudaSuccess) return fail(e);
     if ((e = cudaGraphInstantiate(&graph_loop, g, 0)) != cudaSuccess) return fail(e);
@@ -3567,7 +3576,10 @@ void GpuSolver::solve(SolveStats &stats) {
         CUDA_CHECK(cudaMemcpyAsync(&hs, I.st, sizeof(hs), cudaMemcpyDeviceToHost, I.stream));
         CUDA_CHECK(cudaStreamSynchronize(I.stream));
         const int its = std::max(1, hs.conv_iter >= 0 ? hs.conv_iter + 1 : std::min(hs.iter_base, I.opt.max_iterations));
-        launches += its * (I.kernels_per_iteration() + 1) - (mixed ? 2 * (its - hs.replacements) : 0);
+        if (loop_kind() == LOOP_SINGLE)
+            launches += its * (I.kernels_per_iteration() + 1) - (mixed ? 2 * (its - hs.replacements) : 0);
+        else
+            launches += (its + LOOP_STEP - 1) / LOOP_STEP * (LOOP_STEP * I.kernels_per_iteration() + 1);
     }
     for (int done = 0; !loop && done < I.opt.max_iterations; done += chunk) {
         if (I.opt.use_graph) {
