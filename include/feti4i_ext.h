@@ -203,8 +203,8 @@ void FETI4IElementEnergies(FETI4IInstance instance, FETI4IInt size, const FETI4I
  * and max_order <= 3200; larger values are rejected with an error (return -1,
  * message in FETI4IGetLastError).  A matrix whose order exceeds max_order (or is
  * negative) gets no product: its y range is filled with NaN and *dot is NaN.  The
- * scratch (work-queue counters, one dot partial per matrix) is a static array
- * in device memory, held by every GPU that loads the library until exit; the
+ * scratch (work-queue counters, one item offset per matrix, dot partials) is a
+ * static array in device memory, held by every GPU that loads the library until exit; the
  * first call on a device looks up its address, so that call should come before
  * any stream capture.  Calls share the array: calls that overlap on the GPU
  * race.  stream: a cudaStream_t, or NULL for the default stream. */

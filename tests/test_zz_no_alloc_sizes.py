@@ -1,0 +1,44 @@
+"""FETI4ITiledSymvNoAlloc at the edges of its forms: the one-cluster form and its limit (32 tiles per CTA),
+matrices split into items, ragged and empty orders, many tiny matrices, the product in place."""
+import numpy as np
+import pytest
+
+from espreso_b200 import feti4i as F
+
+pytestmark = pytest.mark.gpu
+
+CASES = {
+    "one_1x1": [1],
+    "one_tile": [32],
+    "ragged_9": [33, 0, 1, 31, 32, 64, 65, 17, 100],
+    "cluster_limit": [224] * 8,              # 28 tiles each: the largest one-cluster call of eight
+    "above_limit": [225] * 8 + [3],
+    "one_large": [1600],
+    "mixed": [7, 1000, 32, 640, 0, 333, 96, 1111],
+    "many_tiny": [5] * 3000,
+}
+
+
+@pytest.mark.parametrize("in_place", [False, True])
+@pytest.mark.parametrize("name", sorted(CASES))
+def test_sizes(name, in_place):
+    import torch
+    rng = np.random.default_rng(len(name))
+    mats = []
+    for n in CASES[name]:
+        A = rng.standard_normal((n, n))
+        mats.append(A + A.T + 3.0 * np.sqrt(n) * np.eye(n))
+    tiles, toff, order = F.pack_symmetric_tiles(mats)
+    voff = np.concatenate([[0], np.cumsum(order)[:-1]]).astype(np.int32)
+    x = rng.standard_normal(int(order.sum()))
+    t = [torch.from_numpy(a).cuda() for a in (tiles, toff, order, voff, x)]
+    y = t[4] if in_place else torch.full((max(1, x.size),), np.nan, dtype=torch.float64, device="cuda")
+    dot = torch.zeros(1, dtype=torch.float64, device="cuda")
+    F.tiled_symv_noalloc(t[0].data_ptr(), t[1].data_ptr(), t[2].data_ptr(), t[3].data_ptr(), order.size,
+                         int(order.max()), t[4].data_ptr(), y.data_ptr(), dot.data_ptr(),
+                         torch.cuda.current_stream().cuda_stream)
+    got = y.cpu().numpy()[:x.size]
+    ref = np.concatenate([S @ x[o:o + n] for S, o, n in zip(mats, voff, order)])
+    # FP64 sums of up to 1600 terms in another order: n eps relative to the norm at most
+    assert np.linalg.norm(got - ref) <= 1600 * 2.3e-16 * np.linalg.norm(ref)
+    assert abs(dot.item() - x @ ref) <= 1600 * 2.3e-16 * np.linalg.norm(x) * np.linalg.norm(ref)
