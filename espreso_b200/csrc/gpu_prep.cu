@@ -113,15 +113,12 @@ __global__ void knorm_kernel(const JobD *jobs, const SubD *subs, const double *a
     const JobD J = jobs[blockIdx.y];
     const SubD sd = subs[J.sub];
     const double *A = arena + sd.a;
-    const long long tot = (long long)J.n * J.n;
     double s = 0.0;
-    for (long long q = (long long)blockIdx.x * blockDim.x + threadIdx.x; q < tot; q += (long long)gridDim.x * blockDim.x) {
-        const int j = (int)(q / J.n), i = (int)(q - (long long)j * J.n);
-        if (i >= j) {
+    for (int j = blockIdx.x; j < J.n; j += gridDim.x)
+        for (int i = j + threadIdx.x; i < J.n; i += blockDim.x) {
             const double v = A[(size_t)j * sd.ld + i];
             s += (i > j ? 2.0 : 1.0) * v * v;
         }
-    }
     __shared__ double red[PT / 32];
     for (int o = 16; o; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
     if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = s;
@@ -136,148 +133,231 @@ __global__ void knorm_kernel(const JobD *jobs, const SubD *subs, const double *a
 // ---------------------------------------------------------------------------------------------
 // elimination step
 
-// Cholesky of the w x w diagonal block of every item, blocked by 32 columns: warp 0 factors a 32 x 32
-// block (one lane per row) and inverts it (one lane per column); all warps multiply the rows below
-// by the inverse and update the rest of the panel block.  A non-positive pivot is recorded (first
-// column per subdomain) and replaced by 1 so that the elimination stays finite.  The inverses of the
-// 32 x 32 diagonal blocks go to `dinv` (four per item) for the panel solve.
+__device__ __forceinline__ void dmma(double (&c)[2], double a, double b) {
+    asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
+                 : "+d"(c[0]), "+d"(c[1])
+                 : "d"(a), "d"(b));
+}
+
+// Cholesky of the w x w diagonal block of every item, blocked by 32 columns.  There is one CTA per
+// subdomain here, so the step is a latency chain: warp 0 factors a 32 x 32 block with its rows in
+// registers (one lane per row, columns passed by shuffles) and inverts it (one lane per column), then all
+// warps multiply the rows below by the inverse and update the rest of the block with FP64 MMAs.
+// (In shared memory, one element at a time, a launch took 200 us on 125 subdomains; 55 us so.)  A
+// non-positive pivot is recorded (first column per subdomain) and replaced by 1 so that the elimination
+// stays finite.  The inverses of the 32 x 32 diagonal blocks go to `dinv` (four per item) for the
+// panel solve.  The block is kept column after column, DLD doubles apart (4 mod 16): the 8 x 4 MMA
+// fragments, the columns and the rows of a 32 x 32 block are all free of bank conflicts.
 constexpr int DB = 32;
-constexpr int DSM = (PW * (PW + 1) + DB * (DB + 1) + (PW - DB) * (DB + 1)) * (int)sizeof(double);
+constexpr int DLD = PW + 4;    // column stride of the diagonal block
+constexpr int VLD = DB + 4;    // column stride of 32-row operands
+constexpr int DSM = (PW * DLD + DB * VLD) * (int)sizeof(double);
 
 __global__ void __launch_bounds__(PT) diag_kernel(const Item *items, const SubD *subs, double *arena, int *fail,
                                                   double *dinv) {
     extern __shared__ double dsm[];
-    double(*D)[PW + 1] = reinterpret_cast<double(*)[PW + 1]>(dsm);
-    double(*V)[DB + 1] = reinterpret_cast<double(*)[DB + 1]>(dsm + PW * (PW + 1));
-    double(*T)[DB + 1] = reinterpret_cast<double(*)[DB + 1]>(dsm + PW * (PW + 1) + DB * (DB + 1));
+    double(*D)[DLD] = reinterpret_cast<double(*)[DLD]>(dsm);                 // D[column][row]
+    double(*V)[VLD] = reinterpret_cast<double(*)[VLD]>(dsm + PW * DLD);      // V[column][row] of the inverse
     __shared__ int s_bad;
     const Item it = items[blockIdx.x];
     const SubD sd = subs[it.sub];
     double *A = arena + sd.a;
     const size_t ld = sd.ld;
     const int k0 = it.k0, w = it.w, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    for (int q = tid; q < w * w; q += PT) {
-        const int i = q % w, j = q / w;
-        if (i >= j) D[i][j] = A[(size_t)(k0 + j) * ld + k0 + i];
+    for (int q = tid; q < PW * w; q += PT) {
+        const int i = q % PW, j = q / PW;
+        if (i >= j && i < w) D[j][i] = A[(size_t)(k0 + j) * ld + k0 + i];
     }
     if (tid == 0) s_bad = -1;
     __syncthreads();
     double *dout = dinv + (size_t)blockIdx.x * (PW / DB) * DB * DB;
+    const int g = lane >> 2, q4 = lane & 3;
     for (int c0 = 0; c0 < w; c0 += DB) {
         const int bw = min(DB, w - c0);
         if (warp == 0) {
-            // factor the bw x bw block, lane = row
-            for (int j = 0; j < bw; ++j) {
-                if (lane == j) {
-                    double d = D[c0 + j][c0 + j];
-                    if (!(d > 0.0)) {
-                        if (s_bad < 0) s_bad = c0 + j;
-                        d = 1.0;
-                    }
-                    D[c0 + j][c0 + j] = sqrt(d);
+            // row `lane` of the block, an identity row beyond bw
+            double a[DB];
+#pragma unroll
+            for (int j = 0; j < DB; ++j)
+                a[j] = (lane < bw && j <= lane) ? D[c0 + j][c0 + lane] : (j == lane ? 1.0 : 0.0);
+            int bad = -1;
+            double rinv = 1.0;   // of the lane's diagonal entry
+#pragma unroll
+            for (int j = 0; j < DB; ++j) {
+                double d = __shfl_sync(0xffffffffu, a[j], j);
+                if (!(d > 0.0)) {
+                    if (bad < 0) bad = c0 + j;
+                    d = 1.0;
                 }
-                __syncwarp();
-                if (lane > j && lane < bw) D[c0 + lane][c0 + j] /= D[c0 + j][c0 + j];
-                __syncwarp();
-                if (lane > j && lane < bw)
-                    for (int c = j + 1; c <= lane; ++c) D[c0 + lane][c0 + c] -= D[c0 + lane][c0 + j] * D[c0 + c][c0 + j];
-                __syncwarp();
+                // 1 / sqrt(d) and sqrt(d), each with a correction step: the square root and the divisions
+                // would be most of the chain
+                double r = rsqrt(d);
+                r = fma(0.5 * r, fma(-d * r, r, 1.0), r);
+                double q = d * r;
+                q = fma(0.5 * r, fma(-q, q, d), q);
+                if (lane == j) rinv = r;
+                a[j] = lane == j ? q : a[j] * r;
+                // (the entries right of a lane's diagonal are never read)
+#pragma unroll
+                for (int c = j + 1; c < DB; ++c) a[c] -= a[j] * __shfl_sync(0xffffffffu, a[j], c);
             }
-            // inverse of the block, lane = column (zero above the diagonal and outside bw)
-            for (int r = 0; r < DB; ++r) V[r][lane] = 0.0;
-            if (lane < bw)
-                for (int r = lane; r < bw; ++r) {
-                    double sum = r == lane ? 1.0 : 0.0;
-                    for (int k = lane; k < r; ++k) sum -= D[c0 + r][c0 + k] * V[k][lane];
-                    V[r][lane] = sum / D[c0 + r][c0 + r];
-                }
+            if (lane == 0 && bad >= 0 && s_bad < 0) s_bad = bad;
+#pragma unroll
+            for (int j = 0; j < DB; ++j)
+                if (lane < bw && j <= lane) D[c0 + j][c0 + lane] = a[j];
             __syncwarp();
-            for (int r = 0; r < DB; ++r) dout[(size_t)(c0 / DB) * DB * DB + r * DB + lane] = V[r][lane];
+            // inverse, lane = column (zero above the diagonal and outside bw)
+            double v[DB];
+#pragma unroll
+            for (int r = 0; r < DB; ++r) {
+                const double ri = __shfl_sync(0xffffffffu, rinv, r);
+                v[r] = 0.0;
+                if (r >= bw) continue;
+                double s0 = r == lane ? 1.0 : 0.0, s1 = 0.0;
+#pragma unroll
+                for (int k = 0; k < r; k += 2) {
+                    s0 -= D[c0 + k][c0 + r] * v[k];
+                    if (k + 1 < r) s1 -= D[c0 + k + 1][c0 + r] * v[k + 1];
+                }
+                v[r] = (s0 + s1) * ri;
+            }
+#pragma unroll
+            for (int r = 0; r < DB; ++r) {
+                const double x = lane < bw ? v[r] : 0.0;
+                V[lane][r] = x;
+                dout[(size_t)(c0 / DB) * DB * DB + r * DB + lane] = x;
+            }
         }
         __syncthreads();
-        // rows below the block within the panel: X = P V^T, X[r][j] = sum_{m <= j} P[r][m] V[j][m]
-        const int rb = c0 + bw, nr = w - rb;
-        for (int q = tid; q < nr * bw; q += PT) {
-            const int r = q % nr, j = q / nr;
-            double sum = 0.0;
-            for (int m = 0; m <= j; ++m) sum += D[rb + r][c0 + m] * V[j][m];
-            T[r][j] = sum;
+        const int rb = c0 + bw, nr = w - rb;   // rows below; bw = 32 when there are any
+        // X = P V^T, eight rows per warp at a time
+        for (int m = warp; 8 * m < nr; m += PT / 32) {
+            const int row = rb + 8 * m;
+            double x[4][2] = {};
+#pragma unroll
+            for (int k = 0; k < DB; k += 4) {
+                const double av = row + g < w ? D[c0 + k + q4][row + g] : 0.0;
+#pragma unroll
+                for (int n = 0; n < 4; ++n)
+                    if (k < 8 * n + 8) dmma(x[n], av, V[k + q4][8 * n + g]);   // V is lower triangular
+            }
+            __syncwarp();
+#pragma unroll
+            for (int n = 0; n < 4; ++n)
+#pragma unroll
+                for (int h = 0; h < 2; ++h)
+                    if (row + g < w) D[c0 + 8 * n + 2 * q4 + h][row + g] = x[n][h];
         }
         __syncthreads();
-        for (int q = tid; q < nr * bw; q += PT) {
-            const int r = q % nr, j = q / nr;
-            D[rb + r][c0 + j] = T[r][j];
-        }
-        __syncthreads();
-        // rest of the panel block: D[i][j] -= sum_m X[i][m] X[j][m], i >= j >= rb
-        for (int q = tid; q < nr * nr; q += PT) {
-            const int i = rb + q % nr, j = rb + q / nr;
-            if (i < j) continue;
-            double sum = 0.0;
-            for (int m = 0; m < bw; ++m) sum += D[i][c0 + m] * D[j][c0 + m];
-            D[i][j] -= sum;
+        // rest of the panel block: D(i, j) -= sum_m X(i, m) X(j, m), 8 x 8 blocks I >= J
+        const int nf = (nr + 7) / 8;
+        for (int f = warp; f < nf * (nf + 1) / 2; f += PT / 32) {
+            int I = (int)((sqrtf(8.0f * f + 1.0f) - 1.0f) * 0.5f);
+            while ((I + 1) * (I + 2) / 2 <= f) ++I;
+            while (I * (I + 1) / 2 > f) --I;
+            const int J = f - I * (I + 1) / 2, ri = rb + 8 * I + g, rj = rb + 8 * J + g;
+            double x[2] = {0.0, 0.0};
+#pragma unroll
+            for (int k = 0; k < DB; k += 4)
+                dmma(x, ri < w ? D[c0 + k + q4][ri] : 0.0, rj < w ? D[c0 + k + q4][rj] : 0.0);
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                const int j = rb + 8 * J + 2 * q4 + h;
+                if (ri < w && j <= ri) D[j][ri] -= x[h];
+            }
         }
         __syncthreads();
     }
     if (tid == 0 && s_bad >= 0) atomicMin(&fail[it.sub], k0 + s_bad);
-    for (int q = tid; q < w * w; q += PT) {
-        const int i = q % w, j = q / w;
-        if (i >= j) A[(size_t)(k0 + j) * ld + k0 + i] = D[i][j];
+    for (int q = tid; q < PW * w; q += PT) {
+        const int i = q % PW, j = q / PW;
+        if (i >= j && i < w) A[(size_t)(k0 + j) * ld + k0 + i] = D[j][i];
     }
 }
 
 // Row blocks below the diagonal block: X = P L_kk^-T by 32-column blocks,
-// X_b = (P_b - sum_{c < b} X_c L_bc^T) V_b^T with the inverted diagonal blocks V_b of diag_kernel.
-constexpr int TSM = (TE * (PW + 1) + DB * (PW + 1) + DB * (DB + 1) + TE * (DB + 1)) * (int)sizeof(double);
+// X_b = (P_b - sum_{c < b} X_c L_bc^T) V_b^T with the inverted diagonal blocks V_b of diag_kernel, on the
+// FP64 tensor-core path: a warp owns eight rows of the block, so only the staging of L and V needs
+// barriers.  (With two shared-memory loads per FMA on the CUDA cores the panel solves took as long as
+// the trailing updates: 382 us a launch on 125 subdomains of 9^3 heat elements,
+// 93 us so.)  A block whose rows are all zero stays zero: K's factor keeps the
+// envelope of the rows, and `nz` (one flag per CTA) lets the trailing update skip its tiles as well.
+constexpr int PLD = TE + 4;    // column stride of the row block
+constexpr int TSM = (PW * PLD + (PW - DB) * VLD + DB * VLD) * (int)sizeof(double);
 
-__global__ void __launch_bounds__(PT) trsm_kernel(const Item *items, int nitems, const SubD *subs, double *arena,
-                                                  const double *dinv) {
+__global__ void __launch_bounds__(PT, 2) trsm_kernel(const Item *items, int nitems, const SubD *subs, double *arena,
+                                                     const double *dinv, int *nz) {
     extern __shared__ double tsm[];
-    double(*P)[PW + 1] = reinterpret_cast<double(*)[PW + 1]>(tsm);
-    double(*Lb)[PW + 1] = reinterpret_cast<double(*)[PW + 1]>(tsm + TE * (PW + 1));
-    double(*V)[DB + 1] = reinterpret_cast<double(*)[DB + 1]>(tsm + (TE + DB) * (PW + 1));
-    double(*T)[DB + 1] = reinterpret_cast<double(*)[DB + 1]>(tsm + (TE + DB) * (PW + 1) + DB * (DB + 1));
-    const int b = blockIdx.x, tid = threadIdx.x;
+    double(*P)[PLD] = reinterpret_cast<double(*)[PLD]>(tsm);                             // P[column][row]
+    double(*L)[VLD] = reinterpret_cast<double(*)[VLD]>(tsm + PW * PLD);                  // L[column][row of block b]
+    double(*V)[VLD] = reinterpret_cast<double(*)[VLD]>(tsm + PW * PLD + (PW - DB) * VLD);
+    const int b = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int ii = find_item<0>(items, nitems, b);
     const Item it = items[ii];
     const SubD sd = subs[it.sub];
     double *A = arena + sd.a;
     const size_t ld = sd.ld;
-    const int k0 = it.k0, w = it.w;
+    const int k0 = it.k0, w = it.w, wp = (w + DB - 1) / DB * DB;
     const int row0 = k0 + w + TE * (b - it.trs0);
     const int rows = min(TE, it.rend - row0);
     const double *vin = dinv + (size_t)ii * (PW / DB) * DB * DB;
-    for (int q = tid; q < TE * w; q += PT) {
+    bool any = false;
+    for (int q = tid; q < TE * wp; q += PT) {
         const int r = q % TE, j = q / TE;
-        P[r][j] = r < rows ? A[(size_t)(k0 + j) * ld + row0 + r] : 0.0;
+        const double v = r < rows && j < w ? A[(size_t)(k0 + j) * ld + row0 + r] : 0.0;
+        P[j][r] = v;
+        any |= v != 0.0;
     }
-    for (int c0 = 0; c0 < w; c0 += DB) {
-        const int bw = min(DB, w - c0);
-        // rows c0.. of the factor block (columns < c0 + bw) and the inverse of its diagonal block
-        for (int q = tid; q < bw * (c0 + bw); q += PT) {
-            const int r = q % bw, c = q / bw;
-            Lb[r][c] = A[(size_t)(k0 + c) * ld + k0 + c0 + r];
+    any = __syncthreads_or(any);
+    if (tid == 0) nz[b] = any;
+    if (!any) return;
+    const int g = lane >> 2, q4 = lane & 3, r = 8 * warp + g;
+    for (int c0 = 0; c0 < wp; c0 += DB) {
+        // rows c0 .. c0 + 31 of the factor block (columns < c0) and the inverse of its diagonal block
+        if (c0 > 0) __syncthreads();
+        for (int q = tid; q < DB * c0; q += PT) {
+            const int n = q % DB, c = q / DB;
+            L[c][n] = c0 + n < w ? A[(size_t)(k0 + c) * ld + k0 + c0 + n] : 0.0;
         }
-        for (int q = tid; q < DB * DB; q += PT) V[q / DB][q % DB] = vin[(size_t)(c0 / DB) * DB * DB + q];
+        for (int q = tid; q < DB * DB; q += PT) V[q % DB][q / DB] = vin[(size_t)(c0 / DB) * DB * DB + q];
         __syncthreads();
-        for (int q = tid; q < TE * bw; q += PT) {
-            const int r = q % TE, m = q / TE;
-            double sum = P[r][c0 + m];
-            for (int c = 0; c < c0; ++c) sum -= P[r][c] * Lb[m][c];
-            T[r][m] = sum;
+        double x[4][2];
+#pragma unroll
+        for (int n = 0; n < 4; ++n)
+#pragma unroll
+            for (int h = 0; h < 2; ++h) x[n][h] = P[c0 + 8 * n + 2 * q4 + h][r];
+        for (int k = 0; k < c0; k += 4) {
+            const double av = -P[k + q4][r];
+#pragma unroll
+            for (int n = 0; n < 4; ++n) dmma(x[n], av, L[k + q4][8 * n + g]);
         }
-        __syncthreads();
-        for (int q = tid; q < TE * bw; q += PT) {
-            const int r = q % TE, j = q / TE;
-            double sum = 0.0;
-            for (int m = 0; m <= j; ++m) sum += T[r][m] * V[j][m];
-            P[r][c0 + j] = sum;
+        __syncwarp();
+#pragma unroll
+        for (int n = 0; n < 4; ++n)
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                P[c0 + 8 * n + 2 * q4 + h][r] = x[n][h];
+                x[n][h] = 0.0;
+            }
+        __syncwarp();
+#pragma unroll
+        for (int k = 0; k < DB; k += 4) {
+            const double av = P[c0 + k + q4][r];
+#pragma unroll
+            for (int n = 0; n < 4; ++n)
+                if (k < 8 * n + 8) dmma(x[n], av, V[k + q4][8 * n + g]);
         }
-        __syncthreads();
+        __syncwarp();
+#pragma unroll
+        for (int n = 0; n < 4; ++n)
+#pragma unroll
+            for (int h = 0; h < 2; ++h) P[c0 + 8 * n + 2 * q4 + h][r] = x[n][h];
+        __syncwarp();
     }
+    __syncthreads();
     for (int q = tid; q < TE * w; q += PT) {
-        const int r = q % TE, j = q / TE;
-        if (r < rows) A[(size_t)(k0 + j) * ld + row0 + r] = P[r][j];
+        const int i = q % TE, j = q / TE;
+        if (i < rows) A[(size_t)(k0 + j) * ld + row0 + i] = P[j][i];
     }
 }
 
@@ -286,12 +366,6 @@ __global__ void __launch_bounds__(PT) trsm_kernel(const Item *items, int nitems,
 // Panels are staged k-major with a stride of 72 doubles (8 mod 16), so the 8 x 4 fragment loads take
 // the minimum of two shared-memory wavefronts.
 constexpr int LDS = 72;
-
-__device__ __forceinline__ void dmma(double (&c)[2], double a, double b) {
-    asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
-                 : "+d"(c[0]), "+d"(c[1])
-                 : "d"(a), "d"(b));
-}
 
 // The panels stream through shared memory in k-chunks of KC with cp.async
 // (two buffers, the next chunk in flight while the current one feeds the MMAs; rows beyond the
@@ -306,7 +380,7 @@ __device__ __forceinline__ void cp_async8(double *dst, const double *src, bool v
 
 template <int KC>
 __global__ void __launch_bounds__(PT, 2) update_pipe_kernel(const Item *items, int nitems, const SubD *subs,
-                                                         double *arena) {
+                                                         double *arena, const int *nz) {
     extern __shared__ double upsm[];
     double(*buf)[2][KC][LDS] = reinterpret_cast<double(*)[2][KC][LDS]>(upsm);   // [stage][panel I / J][k][row]
     const int b = blockIdx.x, tid = threadIdx.x;
@@ -319,6 +393,7 @@ __global__ void __launch_bounds__(PT, 2) update_pipe_kernel(const Item *items, i
     while ((I + 1) * (I + 2) / 2 <= t) ++I;
     while (I * (I + 1) / 2 > t) --I;
     const int J = t - I * (I + 1) / 2;
+    if (!nz[it.trs0 + I] || !nz[it.trs0 + J]) return;   // one of the panels is zero
     const int k0 = it.k0, w = it.w;
     const int r0 = k0 + w;
     const int rI = r0 + TE * I, rJ = r0 + TE * J;
@@ -595,15 +670,19 @@ __global__ void __launch_bounds__(PT) bsolve_kernel(const BItem *items, int nite
             y[r][k] = r < w ? Ys[(size_t)k * it.n + c0 + r] : 0.0;
         }
         __syncthreads();
-        for (int r = w - 1; r >= 0; --r) {
-            if (tid < nk) x[r][tid] = y[r][tid] / D[r][r];
-            __syncthreads();
-            for (int q = tid; q < r * nk; q += PT) {
-                const int i = q % r, k = q / r;
-                y[i][k] -= D[r][i] * x[r][k];
+        // one warp per kernel vector, two rows per lane: no barrier per row
+        if (tid >> 5 < nk) {
+            const int lane = tid & 31, k = tid >> 5;
+            const double i0 = lane < w ? 1.0 / D[lane][lane] : 0.0, i1 = lane + 32 < w ? 1.0 / D[lane + 32][lane + 32] : 0.0;
+            double y0 = y[lane][k], y1 = y[lane + 32][k];
+            for (int r = w - 1; r >= 0; --r) {
+                const double xr = __shfl_sync(0xffffffffu, r < 32 ? y0 * i0 : y1 * i1, r & 31);
+                if (lane < r) y0 -= D[r][lane] * xr;
+                if (lane + 32 < r) y1 -= D[r][lane + 32] * xr;
+                if (lane == 0) x[r][k] = xr;
             }
-            __syncthreads();
         }
+        __syncthreads();
         if (l == below) {
             for (int q = tid; q < w * nk; q += PT) {
                 const int r = q % w, k = q / w;
@@ -793,7 +872,7 @@ void device_factor(const ElementData &el, std::vector<DevFactorJob> &jobs, const
     DevBuf<double> arena, stage, fxb, vals, bsign, reg, part, dX, dY, dinvb;
     DevBuf<TJob> dtj;
     DevBuf<BItem> dbi;
-    DevBuf<int> epos, bpos, fail, list;
+    DevBuf<int> epos, bpos, fail, list, nzb;
     DevBuf<SubD> dsubs;
     DevBuf<JobD> djobs;
     DevBuf<ElemD> dels;
@@ -972,8 +1051,13 @@ void device_factor(const ElementData &el, std::vector<DevFactorJob> &jobs, const
         std::vector<size_t> o1 = offsets(ph1), o2 = offsets(ph2), o3 = offsets(ph3);
         ditems.put(all);
         size_t maxitems = 0;   // inverted 32 x 32 diagonal blocks of the largest step
+        int maxtrs = 1;        // row blocks of the largest step
         for (auto *ph : {&ph1, &ph2, &ph3})
-            for (auto &st : *ph) maxitems = std::max(maxitems, st.items.size());
+            for (auto &st : *ph) {
+                maxitems = std::max(maxitems, st.items.size());
+                maxtrs = std::max(maxtrs, st.ntrs);
+            }
+        nzb.reserve(maxtrs);
         dinvb.reserve(std::max<size_t>(maxitems, 1) * (PW / DB) * DB * DB);
         tm.flops += flops;
 
@@ -1005,11 +1089,11 @@ void device_factor(const ElementData &el, std::vector<DevFactorJob> &jobs, const
                 diag_kernel<<<ni, PT, DSM>>>(it, dsubs.p, arena.p, fail.p, dinvb.p);
                 ++tm.launches;
                 if (ph[s].ntrs > 0) {
-                    trsm_kernel<<<ph[s].ntrs, PT, TSM>>>(it, ni, dsubs.p, arena.p, dinvb.p);
+                    trsm_kernel<<<ph[s].ntrs, PT, TSM>>>(it, ni, dsubs.p, arena.p, dinvb.p, nzb.p);
                     ++tm.launches;
                 }
                 if (ph[s].nupd > 0) {
-                    update_pipe_kernel<16><<<ph[s].nupd, PT, UPSM16>>>(it, ni, dsubs.p, arena.p);
+                    update_pipe_kernel<16><<<ph[s].nupd, PT, UPSM16>>>(it, ni, dsubs.p, arena.p, nzb.p);
                     ++tm.launches;
                 }
             }
