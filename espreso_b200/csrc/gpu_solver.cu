@@ -105,7 +105,9 @@ struct BlockDev {
     int lg;              // log2(nr)
     double *x, *r, *w, *z, *y, *p, *Ap, *Ax, *bL, *uT, *vT, *d, *alpha, *e;
     float *p32;          // FP32 copy of p (SYMM input in mixed precision)
-    double *part;        // nd * nr partials
+    double *part;        // partials of the totals: one row of nr per CTA or subdomain
+    double *part2;       // DONE_COUNT x GT_GROUPS x nr partials of the CTA groups
+    int *gdone;          // DONE_COUNT x GT_GROUPS completion counters of the groups
     double *unit_dot;    // SYMM work units * nr
     double *scal;        // SC_COUNT * nr
     double *rho_hist;    // (max_it + 64) * nr
@@ -2046,6 +2048,14 @@ __global__ void hyb_kr_kernel(DevProblem P, HybDev H, const int *doff, const int
 }  // namespace
 
 // =============================================================================================
+// f(integral constant) with the kernel width of the problem
+template <typename F>
+static void with_kwidth(int KS, F &&f) {
+    if (KS == 1) f(std::integral_constant<int, 1>());
+    else if (KS == 6) f(std::integral_constant<int, 6>());
+    else f(std::integral_constant<int, 0>());
+}
+
 constexpr int kSizeClasses = 5;
 
 struct TileSetHost {
@@ -2153,6 +2163,7 @@ struct GpuSolver::Impl {
         double *rhs = nullptr, *sol = nullptr, *f = nullptr, *kf = nullptr, *g = nullptr;
         double *zk = nullptr;   // forward results L^-1 f of every column (K^+ modes 1 and 2)
         int flat_grid = 1;
+        int cluster = 1;          // CTAs per subdomain of bz, bupdate
         int2 *units4 = nullptr;
         int nunits4 = 0;
         float *pan = nullptr;          // K-major panels of the mixed blocks (asynchronous tensor-core SYMM)
@@ -2953,14 +2964,6 @@ static void set_smem_limits() {
     w_limits(std::integral_constant<int, 1>());
     w_limits(std::integral_constant<int, 6>());
     done = true;
-}
-
-// f(integral constant) with the kernel width of the problem
-template <typename F>
-static void with_kwidth(int KS, F &&f) {
-    if (KS == 1) f(std::integral_constant<int, 1>());
-    else if (KS == 6) f(std::integral_constant<int, 6>());
-    else f(std::integral_constant<int, 0>());
 }
 
 void GpuSolver::Impl::launch_r0(int replace_mode, int slot) {
@@ -4210,33 +4213,50 @@ __device__ void block_sum_cols(double v, int nr, double *sh /* >= 8*32 */, doubl
     __syncthreads();
 }
 
-// last-CTA total of per-CTA column partials (partials[cta * nr + j]) into out[j]
-__device__ void grid_total_cols(const double *mine /* nr, shared */, double *partials, int nr, int *counter,
-                                double *out) {
+// Totals of the CTAs' column partials (partials[cta * nr + j]) into out[j], in a fixed order.  The last
+// CTA of a group of CTAs sums the group, the last group sums the groups: a single last CTA over the 592
+// to 1,776 of a kernel runs on for several microseconds after the others.
+constexpr int GT_GROUPS = 64;
+__device__ void grid_total_cols(const double *mine /* nr, shared */, double *partials, const BlockDev &B, int id, double *out) {
     __shared__ int s_last;
-    __syncthreads();
-    if (threadIdx.x < nr) partials[blockIdx.x * nr + threadIdx.x] = mine[threadIdx.x];
-    __threadfence();
-    __syncthreads();
-    if (threadIdx.x == 0) s_last = (atomicAdd(counter, 1) == (int)gridDim.x - 1);
-    __syncthreads();
-    if (s_last) {
-        // every thread of the last CTA sums a fixed subset of the CTA partials of one column,
-        // then the subsets are combined in shared memory (fixed order: deterministic)
-        __threadfence();
-        __shared__ double s_cols[1024];
-        const int j = threadIdx.x & (nr - 1), g = threadIdx.x / nr, ng = blockDim.x / nr;
+    __shared__ double s_cols[1024];
+    const int nr = B.nr, row = blockIdx.x, nrows = gridDim.x;
+    const int gs = max(32, (nrows + GT_GROUPS - 1) / GT_GROUPS), ngr = (nrows + gs - 1) / gs;
+    const int grp = row / gs, first = grp * gs, cnt = min(gs, nrows - first);
+    int *gcount = B.gdone + id * GT_GROUPS + grp;
+    double *part2 = B.part2 + (size_t)id * GT_GROUPS * nr;
+    const int j = threadIdx.x & (nr - 1), g = threadIdx.x / nr, ng = blockDim.x / nr;
+    auto sum = [&](const double *v, int n, double *to) {   // to[j] = sum of n rows of v
         double t = 0.0;
-        for (int c = g; c < (int)gridDim.x; c += ng) t += __ldcg(&partials[c * nr + j]);
+        for (int c = g; c < n; c += ng) t += __ldcg(&v[(size_t)c * nr + j]);
         s_cols[threadIdx.x] = t;
         __syncthreads();
         if (threadIdx.x < nr) {
             double u = 0.0;
             for (int q = 0; q < ng; ++q) u += s_cols[q * nr + threadIdx.x];
-            out[threadIdx.x] = u;
+            to[threadIdx.x] = u;
         }
-        if (threadIdx.x == 0) *counter = 0;
+    };
+    __syncthreads();
+    if (threadIdx.x < nr) partials[(size_t)row * nr + threadIdx.x] = mine[threadIdx.x];
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) s_last = (atomicAdd(gcount, 1) == cnt - 1);
+    __syncthreads();
+    if (!s_last) return;
+    __threadfence();
+    sum(partials + (size_t)first * nr, cnt, part2 + (size_t)grp * nr);
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        *gcount = 0;
+        s_last = (atomicAdd(B.done + id, 1) == ngr - 1);
     }
+    __syncthreads();
+    if (!s_last) return;
+    __threadfence();
+    sum(part2, ngr, out);
+    if (threadIdx.x == 0) B.done[id] = 0;
 }
 
 // G_i v per column, v[(e - e0) * nr + j] (rows of the subdomain, written by this CTA)
@@ -4254,21 +4274,47 @@ __device__ void g_dot_cols(const DevProblem &P, const BlockDev &B, int dsub, con
     }
 }
 
-// G_i v per column from per-thread partial sums gk[k] = sum over the thread's elements of
-// G[e, k] v[e, j] (every thread of the CTA on one column j = threadIdx.x & (nr - 1)): one pass over
-// the rows instead of one per kernel vector
+// G_i v per column from per-thread partial sums gk[k] = sum over the thread's rows of G[e, k] v[e, j..j+1]
+// (every thread on the columns j = 2 (threadIdx.x mod nr/2) and j + 1, 256 threads per CTA), over the CTAs
+// of the subdomain's cluster in rank order.  After cluster_enter.
 template <int KC>
-__device__ void g_cols_reduce(const DevProblem &P, const BlockDev &B, int dsub, double (&gk)[KC], double *sh) {
-    __shared__ double cols[32];
-    const int nk = P.kof[dsub + 1] - P.kof[dsub];
+__device__ void g_cols_finish(const DevProblem &P, const BlockDev &B, int dsub, double2 (&gk)[KC]) {
+    __shared__ double sh[8 * KC * 32];
+    __shared__ double cl[8 * KC * 32];
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nr = B.nr, hn = nr >> 1;
+    const unsigned C = cluster_size_x(), rank = cluster_rank_x();
 #pragma unroll
     for (int k = 0; k < KC; ++k) {
-        if (k < nk) {   // uniform over the CTA
-            block_sum_cols(gk[k], B.nr, sh, cols);
-            if (threadIdx.x < B.nr) B.d[(size_t)(P.kof[dsub] + k) * B.nr + threadIdx.x] = cols[threadIdx.x];
-            __syncthreads();
+        for (int o = 16; o >= hn; o >>= 1) {
+            gk[k].x += __shfl_xor_sync(FULL, gk[k].x, o);
+            gk[k].y += __shfl_xor_sync(FULL, gk[k].y, o);
+        }
+        if (lane < hn) {
+            sh[(wid * KC + k) * 32 + 2 * lane] = gk[k].x;
+            sh[(wid * KC + k) * 32 + 2 * lane + 1] = gk[k].y;
         }
     }
+    __syncthreads();
+    cluster_entered();
+    const int nk = P.kof[dsub + 1] - P.kof[dsub];
+    double *out = B.d + (size_t)P.kof[dsub] * nr;
+    for (int q = threadIdx.x; q < nk * nr; q += blockDim.x) {
+        const int k = q >> B.lg, j = q & (nr - 1);
+        double t = 0.0;
+#pragma unroll
+        for (int w = 0; w < 8; ++w) t += sh[(w * KC + k) * 32 + j];
+        if (C > 1) st_cluster(&cl[(rank * KC + k) * 32 + j], 0, t);
+        else out[q] = t;
+    }
+    if (C == 1) return;
+    cluster_arrive();
+    cluster_wait();
+    if (rank == 0)
+        for (int q = threadIdx.x; q < nk * nr; q += blockDim.x) {
+            double t = 0.0;
+            for (unsigned r = 0; r < C; ++r) t += cl[(r * KC + (q >> B.lg)) * 32 + (q & (nr - 1))];
+            out[q] = t;
+        }
 }
 
 __device__ __forceinline__ double gt_alpha_col(const DevProblem &P, int e, int j, int nr, const double *a) {
@@ -4368,7 +4414,7 @@ __global__ void br0_kernel(DevProblem P, BlockDev B, int replace_mode, int slot)
     g_dot_cols(P, B, dsub, B.r + (size_t)e0 * nr, sh);
     if (!replace_mode) {
         block_sum_cols(bb, nr, sh, cols);
-        grid_total_cols(cols, B.part, nr, B.done + DONE_B, B.scal + SC_BN2 * nr);
+        grid_total_cols(cols, B.part, B, DONE_B, B.scal + SC_BN2 * nr);
     }
 }
 
@@ -4383,7 +4429,7 @@ __global__ void bpnorm_kernel(DevProblem P, BlockDev B) {
         s += u * u * P.minv[e];
     }
     block_sum_cols(s, nr, sh, cols);
-    grid_total_cols(cols, B.part, nr, B.done + DONE_PN, B.scal + SC_PN2 * nr);
+    grid_total_cols(cols, B.part, B, DONE_PN, B.scal + SC_PN2 * nr);
 }
 
 __global__ void btol_kernel(DevProblem P, BlockDev B) {
@@ -4394,51 +4440,6 @@ __global__ void btol_kernel(DevProblem P, BlockDev B) {
         B.rmax[j] = un;
         B.conv[j] = (bn == 0.0 || un == 0.0) ? -2 : -1;
     }
-}
-
-// KC: the kernel width (1, 6: G z accumulated in registers while z is formed; 0: per-row counts,
-// a second pass over z)
-template <int KC>
-__global__ void __launch_bounds__(TPBB) bz_kernel(DevProblem P, BlockDev B, int slot) {
-    pdl_enter();
-    __shared__ double sh[32 * 32];
-    const int iter = P.st->iter_base + slot;
-    if (skip_iter(P.st, iter)) return;
-    const int nr = B.nr, dsub = blockIdx.x;
-    const int e0 = P.loff[dsub], e1 = P.loff[dsub + 1];
-    const int cnt = (e1 - e0) * nr;
-    constexpr int NG = KC > 0 ? KC : 1;
-    double gk[NG];
-#pragma unroll
-    for (int k = 0; k < NG; ++k) gk[k] = 0.0;
-    for (int i0 = threadIdx.x; i0 < cnt; i0 += UNR * blockDim.x) {
-        double zv[UNR];
-#pragma unroll
-        for (int u = 0; u < UNR; ++u) {
-            const int i = i0 + u * blockDim.x;
-            if (i < cnt) {
-                const int e = e0 + (i >> B.lg), j = i & (nr - 1);
-                const int pt = P.ptidx[e];
-                zv[u] = P.ws[e] * B.vT[(size_t)P.tidx[e] * nr + j];
-                if (pt >= 0) zv[u] += P.pws[e] * B.vT[(size_t)pt * nr + j];
-            }
-        }
-#pragma unroll
-        for (int u = 0; u < UNR; ++u) {
-            const int i = i0 + u * blockDim.x;
-            if (i < cnt) {
-                B.z[(size_t)e0 * nr + i] = zv[u];
-                if (KC > 0) {
-                    const double *g = P.Gl + (size_t)(e0 + (i >> B.lg)) * NG;
-#pragma unroll
-                    for (int k = 0; k < NG; ++k) gk[k] += __ldg(g + k) * zv[u];
-                }
-            }
-        }
-    }
-    __syncthreads();
-    if (KC > 0) g_cols_reduce<NG>(P, B, dsub, gk, sh);
-    else g_dot_cols(P, B, dsub, B.z + (size_t)e0 * nr, sh);
 }
 
 // ---- flat block kernels: a persistent grid over all rows (no per-subdomain reduction needed)
@@ -4507,6 +4508,80 @@ __device__ __forceinline__ double2 gt_alpha_colk2(const DevProblem &P, int e, in
         r.y += g[k] * x.y + gp[k] * y.y;
     }
     return r;
+}
+
+// z = assemble(W B v_T), d = G z and rho_j = z.w, which is y.w for y = P z because w = P r lies in the range
+// of the projector: with rho known here, y and p = y + beta p are formed in one pass (byp_flat2).
+// KC: the kernel width (1, 6: G z accumulated in registers while z is formed; 0: per-row counts,
+// a second pass over z).  A cluster of CTAs per subdomain, two columns per thread.
+template <int KC>
+__global__ void __launch_bounds__(256, KC == 6 ? 4 : 6) bz_kernel(DevProblem P, BlockDev B, int slot) {
+    constexpr int UNR = 2;
+    pdl_enter();
+    __shared__ double sh[8 * 32];
+    __shared__ double cols[32];
+    const int iter = P.st->iter_base + slot;
+    if (skip_iter(P.st, iter)) return;
+    cluster_enter();
+    const int C = (int)cluster_size_x(), dsub = blockIdx.x / C;
+    const int nr = B.nr, hn = nr >> 1, lh = B.lg - 1;
+    const int e0 = P.loff[dsub], e1 = P.loff[dsub + 1], cnt = (e1 - e0) * hn;
+    constexpr int NG = KC > 0 ? KC : 1;
+    double2 gk[NG];
+#pragma unroll
+    for (int k = 0; k < NG; ++k) gk[k] = make_double2(0.0, 0.0);
+    double s0 = 0.0, s1 = 0.0;
+    const double2 *vT = reinterpret_cast<const double2 *>(B.vT);
+    const double2 *w = reinterpret_cast<const double2 *>(B.w) + (size_t)e0 * hn;
+    double2 *z = reinterpret_cast<double2 *>(B.z) + (size_t)e0 * hn;
+    const int step = C * blockDim.x, jh = threadIdx.x & (hn - 1);
+    for (int i0 = cluster_rank_x() * blockDim.x + threadIdx.x; i0 < cnt; i0 += UNR * step) {
+        double2 v[UNR], wv[UNR];
+        double mv[UNR];
+#pragma unroll
+        for (int u = 0; u < UNR; ++u) {
+            const int i = i0 + u * step;
+            if (i < cnt) {
+                const int e = e0 + (i >> lh), pt = __ldg(P.ptidx + e);
+                const double a = __ldg(P.ws + e), c = __ldg(P.pws + e);
+                const double2 x = __ldg(vT + (size_t)__ldg(P.tidx + e) * hn + jh);
+                // a row without a partner has pws 0; its own T row stands in for the partner's
+                const double2 y = __ldg(vT + (size_t)(pt >= 0 ? pt : __ldg(P.tidx + e)) * hn + jh);
+                v[u] = make_double2(a * x.x, a * x.y);
+                if (pt >= 0) {
+                    v[u].x += c * y.x;
+                    v[u].y += c * y.y;
+                }
+                wv[u] = __ldg(w + i);
+                mv[u] = __ldg(P.minv + e);
+            }
+        }
+#pragma unroll
+        for (int u = 0; u < UNR; ++u) {
+            const int i = i0 + u * step;
+            if (i < cnt) {
+                z[i] = v[u];
+                s0 += v[u].x * wv[u].x * mv[u];
+                s1 += v[u].y * wv[u].y * mv[u];
+                if (KC > 0) {
+                    const double *g = P.Gl + (size_t)(e0 + (i >> lh)) * NG;
+#pragma unroll
+                    for (int k = 0; k < NG; ++k) {
+                        gk[k].x += __ldg(g + k) * v[u].x;
+                        gk[k].y += __ldg(g + k) * v[u].y;
+                    }
+                }
+            }
+        }
+    }
+    if (KC > 0) {
+        g_cols_finish<NG>(P, B, dsub, gk);
+    } else {
+        __syncthreads();
+        g_dot_cols(P, B, dsub, B.z + (size_t)e0 * nr, sh);
+    }
+    block_sum_cols2(s0, s1, nr, sh, cols);
+    grid_total_cols(cols, B.part, B, DONE_RHO, B.scal + SC_RHO * nr);
 }
 
 __global__ void __launch_bounds__(256, FLAT_MIN_BLOCKS) bell_flat2_kernel(DevProblem P, BlockDev B, int slot) {
@@ -4588,9 +4663,9 @@ __global__ void __launch_bounds__(256, FLAT_MIN_BLOCKS) bw_flat2_kernel(DevProbl
         }
     }
     block_sum_cols2(s0, s1, nr, sh, cols);
-    grid_total_cols(cols, B.part, nr, B.done + DONE_W, B.scal + SC_WN2 * nr);
+    grid_total_cols(cols, B.part, B, DONE_W, B.scal + SC_WN2 * nr);
     if (PRECOND == PREC_NONE)
-        grid_total_cols(cols, B.part + (size_t)gridDim.x * nr, nr, B.done + DONE_RHO, B.scal + SC_RHO * nr);
+        grid_total_cols(cols, B.part + (size_t)gridDim.x * nr, B, DONE_RHO, B.scal + SC_RHO * nr);
 }
 
 // w = r - G^T alpha and u_T = B^T W w in one pass over the touched DOFs: a thread takes one T entry
@@ -4628,53 +4703,53 @@ __global__ void __launch_bounds__(256, FLAT_MIN_BLOCKS) bwu_flat2_kernel(DevProb
         if (PRECOND == PREC_WEIGHT) *reinterpret_cast<double2 *>(B.vT + (size_t)t * nr + j) = u;
     }
     block_sum_cols2(s0, s1, nr, sh, cols);
-    grid_total_cols(cols, B.part, nr, B.done + DONE_W, B.scal + SC_WN2 * nr);
+    grid_total_cols(cols, B.part, B, DONE_W, B.scal + SC_WN2 * nr);
 }
 
+// p = (z - G^T alpha) + beta_j p and its FP32 copy: y = P z is not stored.  Two columns per thread; the grid
+// stride is a multiple of nr / 2, so every thread keeps its columns and computes their beta once.
+// (As two kernels with y written and read back, and w read for rho: 92 + 51 us for 512 subdomains of
+// 10^3 heat elements and 32 columns; 68 us so.)
 template <int KC>
-__global__ void __launch_bounds__(256, FLAT_MIN_BLOCKS) by_flat2_kernel(DevProblem P, BlockDev B, int slot) {
+__global__ void __launch_bounds__(256, FLAT_MIN_BLOCKS) byp_flat2_kernel(DevProblem P, BlockDev B, int slot) {
     pdl_enter();
-    __shared__ double sh[8 * 32];
-    __shared__ double cols[32];
     const int iter = P.st->iter_base + slot;
     if (skip_iter(P.st, iter)) return;
-    const int nr = B.nr, lh = B.lg - 1;
-    const long long cnt = (long long)P.NL * (nr >> 1), stride = (long long)gridDim.x * blockDim.x;
-    double s0 = 0.0, s1 = 0.0;
-    for (long long i0 = (long long)blockIdx.x * blockDim.x + threadIdx.x; i0 < cnt; i0 += UNR * stride) {
-        double2 zv[UNR], ga[UNR], wv[UNR];
-        double mv[UNR];
+    const int nr = B.nr, hn = nr >> 1, lh = B.lg - 1;
+    const long long cnt = (long long)P.NL * hn, stride = (long long)gridDim.x * blockDim.x;
+    const long long i0 = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    const int j = 2 * (int)(i0 & (hn - 1));
+    const bool f0 = col_frozen(B, j, iter), f1 = col_frozen(B, j + 1, iter);
+    const double b0 = (iter == 0) ? 0.0 : B.scal[SC_RHO * nr + j] / B.rho_hist[(size_t)(iter - 1) * nr + j];
+    const double b1 = (iter == 0) ? 0.0 : B.scal[SC_RHO * nr + j + 1] / B.rho_hist[(size_t)(iter - 1) * nr + j + 1];
+    const double2 *z = reinterpret_cast<const double2 *>(B.z);
+    double2 *p = reinterpret_cast<double2 *>(B.p);
+    float2 *p32 = reinterpret_cast<float2 *>(B.p32);
+    for (long long i = i0; i < cnt; i += UNR * stride) {
+        double2 zv[UNR], pv[UNR], ga[UNR];
 #pragma unroll
         for (int u = 0; u < UNR; ++u) {
-            const long long i = i0 + u * stride;
-            if (i < cnt) {
-                const int e = (int)(i >> lh), j = 2 * (int)(i & ((nr >> 1) - 1));
-                const size_t o = (size_t)e * nr + j;
-                zv[u] = *reinterpret_cast<const double2 *>(B.z + o);
-                wv[u] = *reinterpret_cast<const double2 *>(B.w + o);
-                ga[u] = gt_alpha_colk2<KC>(P, e, j, nr, B.alpha);
-                mv[u] = P.minv[e];
+            const long long k = i + u * stride;
+            if (k < cnt) {
+                zv[u] = __ldg(z + k);
+                pv[u] = p[k];
+                ga[u] = gt_alpha_colk2<KC>(P, (int)(k >> lh), j, nr, B.alpha);
             }
         }
 #pragma unroll
         for (int u = 0; u < UNR; ++u) {
-            const long long i = i0 + u * stride;
-            if (i < cnt) {
-                const int e = (int)(i >> lh), j = 2 * (int)(i & ((nr >> 1) - 1));
-                const double2 yv = make_double2(zv[u].x - ga[u].x, zv[u].y - ga[u].y);
-                *reinterpret_cast<double2 *>(B.y + (size_t)e * nr + j) = yv;
-                s0 += yv.x * wv[u].x * mv[u];
-                s1 += yv.y * wv[u].y * mv[u];
+            const long long k = i + u * stride;
+            if (k < cnt) {
+                const double2 r = make_double2(f0 ? 0.0 : (zv[u].x - ga[u].x) + b0 * pv[u].x,
+                                               f1 ? 0.0 : (zv[u].y - ga[u].y) + b1 * pv[u].y);
+                p[k] = r;
+                p32[k] = make_float2((float)r.x, (float)r.y);
             }
         }
     }
-    block_sum_cols2(s0, s1, nr, sh, cols);
-    grid_total_cols(cols, B.part + (size_t)gridDim.x * nr, nr, B.done + DONE_RHO, B.scal + SC_RHO * nr);
 }
 
-
-// y = z - G^T alpha, rho_j = y.w
-
+// The same without a preconditioner, where y = w is already there:
 // p = y + beta_j p (and its FP32 copy).  Two columns per thread (16-byte loads and stores), UNR
 // rows in flight; the grid stride is a multiple of nr / 2, so every thread keeps its columns and
 // computes their beta once.
@@ -4714,69 +4789,75 @@ __global__ void __launch_bounds__(256, FLAT_MIN_BLOCKS) bp_kernel(DevProblem P, 
     }
 }
 
-// Two CTAs of 1024 threads per SM (32 registers, two rows in flight per thread): with 60 registers
-// only one fitted, and the 512 subdomains of the heat workload ran in four waves.
+// x += alpha_j p, r -= alpha_j assemble(Ap), d = G r, convergence check per column.  A cluster of CTAs per
+// subdomain, two columns per thread (16-byte accesses).  One CTA of 1024 threads per subdomain filled the
+// chip in 1.7 waves with 512 subdomains (121 us at 32 columns, 116 us so: 0.69 GB of vectors) and less than
+// half of it with 64 (44 us at 16 columns, 19 us so).
 template <int KC>
-__global__ void __launch_bounds__(TPBB, 2) bupdate_kernel(DevProblem P, BlockDev B, int slot) {
+__global__ void __launch_bounds__(256, 4) bupdate_kernel(DevProblem P, BlockDev B, int slot) {
     constexpr int UNR = 2;
     constexpr int NG = KC > 0 ? KC : 1;
-    double gk[NG];
-#pragma unroll
-    for (int k = 0; k < NG; ++k) gk[k] = 0.0;
     pdl_enter();
-    __shared__ double sh[32 * 32];
+    __shared__ double sh[8 * 32];
     const int iter = P.st->iter_base + slot;
     if (skip_iter(P.st, iter)) return;
-    const int nr = B.nr, dsub = blockIdx.x;
-    const int e0 = P.loff[dsub], e1 = P.loff[dsub + 1];
-    // the stride keeps each thread on one column: alpha_j once per thread
-    const int jt = threadIdx.x & (nr - 1);
-    const bool frozen = col_frozen(B, jt, iter);
-    const double alpha = frozen ? 0.0 : B.scal[SC_RHO * nr + jt] / B.scal[SC_PAP * nr + jt];
-    const int cnt = (e1 - e0) * nr;
-    if (!frozen)
-        for (int i0 = threadIdx.x; i0 < cnt; i0 += UNR * blockDim.x) {
-            double xv[UNR], pv[UNR], rv[UNR], av[UNR];
+    cluster_enter();
+    const int C = (int)cluster_size_x(), dsub = blockIdx.x / C;
+    const int nr = B.nr, hn = nr >> 1, lh = B.lg - 1;
+    const int e0 = P.loff[dsub], e1 = P.loff[dsub + 1], cnt = (e1 - e0) * hn;
+    // the stride keeps each thread on its two columns: alpha_j once per thread, 0 for a converged column,
+    // which keeps its x and r (its G r is still the coarse input of the next iteration)
+    const int jh = threadIdx.x & (hn - 1), j = 2 * jh;
+    const double al0 = col_frozen(B, j, iter) ? 0.0 : B.scal[SC_RHO * nr + j] / B.scal[SC_PAP * nr + j];
+    const double al1 = col_frozen(B, j + 1, iter) ? 0.0 : B.scal[SC_RHO * nr + j + 1] / B.scal[SC_PAP * nr + j + 1];
+    double2 gk[NG];
 #pragma unroll
-            for (int u = 0; u < UNR; ++u) {
-                const int i = i0 + u * blockDim.x;
-                if (i < cnt) {
-                    const int e = e0 + (i >> B.lg);
-                    const size_t o = (size_t)e0 * nr + i;
-                    const int q = P.partner[e];
-                    xv[u] = B.x[o];
-                    pv[u] = B.p[o];
-                    rv[u] = B.r[o];
-                    av[u] = B.Ap[o] + (q >= 0 ? B.Ap[(size_t)q * nr + jt] : 0.0);
+    for (int k = 0; k < NG; ++k) gk[k] = make_double2(0.0, 0.0);
+    const double2 *Ap = reinterpret_cast<const double2 *>(B.Ap), *p = reinterpret_cast<const double2 *>(B.p) + (size_t)e0 * hn;
+    double2 *x = reinterpret_cast<double2 *>(B.x) + (size_t)e0 * hn, *r = reinterpret_cast<double2 *>(B.r) + (size_t)e0 * hn;
+    const int step = C * blockDim.x;
+    for (int i0 = cluster_rank_x() * blockDim.x + threadIdx.x; i0 < cnt; i0 += UNR * step) {
+        double2 xv[UNR], pv[UNR], rv[UNR], av[UNR];
+#pragma unroll
+        for (int u = 0; u < UNR; ++u) {
+            const int i = i0 + u * step;
+            if (i < cnt) {
+                const int q = __ldg(P.partner + e0 + (i >> lh));
+                xv[u] = x[i];
+                pv[u] = __ldg(p + i);
+                rv[u] = r[i];
+                av[u] = __ldg(Ap + (size_t)e0 * hn + i);
+                if (q >= 0) {
+                    const double2 b = __ldg(Ap + (size_t)q * hn + jh);
+                    av[u].x += b.x;
+                    av[u].y += b.y;
                 }
             }
+        }
 #pragma unroll
-            for (int u = 0; u < UNR; ++u) {
-                const int i = i0 + u * blockDim.x;
-                if (i < cnt) {
-                    const size_t o = (size_t)e0 * nr + i;
-                    B.x[o] = xv[u] + alpha * pv[u];
-                    const double rn = rv[u] - alpha * av[u];
-                    B.r[o] = rn;
-                    if (KC > 0) {
-                        const double *g = P.Gl + (size_t)(e0 + (i >> B.lg)) * NG;
+        for (int u = 0; u < UNR; ++u) {
+            const int i = i0 + u * step;
+            if (i < cnt) {
+                x[i] = make_double2(xv[u].x + al0 * pv[u].x, xv[u].y + al1 * pv[u].y);
+                const double2 rn = make_double2(rv[u].x - al0 * av[u].x, rv[u].y - al1 * av[u].y);
+                r[i] = rn;
+                if (KC > 0) {
+                    const double *g = P.Gl + (size_t)(e0 + (i >> lh)) * NG;
 #pragma unroll
-                        for (int k = 0; k < NG; ++k) gk[k] += __ldg(g + k) * rn;
+                    for (int k = 0; k < NG; ++k) {
+                        gk[k].x += __ldg(g + k) * rn.x;
+                        gk[k].y += __ldg(g + k) * rn.y;
                     }
                 }
             }
         }
-    else if (KC > 0)
-        // a converged column keeps its r: its G r is still the coarse input of the next iteration
-        for (int i = threadIdx.x; i < cnt; i += blockDim.x) {
-            const double *g = P.Gl + (size_t)(e0 + (i >> B.lg)) * NG;
-            const double rv = B.r[(size_t)e0 * nr + i];
-#pragma unroll
-            for (int k = 0; k < NG; ++k) gk[k] += __ldg(g + k) * rv;
-        }
-    __syncthreads();
-    if (KC > 0) g_cols_reduce<NG>(P, B, dsub, gk, sh);
-    else g_dot_cols(P, B, dsub, B.r + (size_t)e0 * nr, sh);
+    }
+    if (KC > 0) {
+        g_cols_finish<NG>(P, B, dsub, gk);
+    } else {
+        __syncthreads();
+        g_dot_cols(P, B, dsub, B.r + (size_t)e0 * nr, sh);
+    }
     if (blockIdx.x == 0 && threadIdx.x == 0) {
         DevState *st = P.st;
         bool replace = false;
@@ -6203,7 +6284,13 @@ void GpuSolver::Impl::ensure_block(int nr) {
     // persistent grid of the flat block kernels: rows of all subdomains, UNR per thread in flight
     blk.flat_grid =
         std::max(1, std::min(nsm * FLAT_MIN_BLOCKS, (int)(((long long)NL * nr + 256LL * UNR - 1) / (256LL * UNR))));
-    B.part = alloc<double>((size_t)2 * std::max(nd, blk.flat_grid) * nr);
+    // subdomain kernels: up to 8 CTAs per subdomain while there are fewer than six per SM
+    blk.cluster = 1;
+    while (blk.cluster < 8 && blk.cluster * nd < 6 * nsm) blk.cluster *= 2;
+    B.part = alloc<double>((size_t)2 * std::max(nd * blk.cluster, blk.flat_grid) * nr);
+    B.part2 = alloc<double>((size_t)DONE_COUNT * GT_GROUPS * nr);
+    B.gdone = alloc<int>(DONE_COUNT * GT_GROUPS);
+    CUDA_CHECK(cudaMemset(B.gdone, 0, sizeof(int) * DONE_COUNT * GT_GROUPS));
     B.scal = alloc<double>((size_t)SC_COUNT * nr);
     B.rho_hist = alloc<double>((size_t)(opt.max_iterations + 64) * nr);
     B.tol = alloc<double>(nr); B.rmax = alloc<double>(nr); B.last_norm = alloc<double>(nr);
@@ -6527,27 +6614,24 @@ void GpuSolver::Impl::launch_block_iteration(int slot) {
 #undef BWU
 #undef BW
     if (opt.precond != PREC_NONE) {
-        switch (P.KS) {
-        case 1: launch_pdl(bz_kernel<1>, dim3(nd), dim3(TPBB), 0, stream, P, B, slot); break;
-        case 6: launch_pdl(bz_kernel<6>, dim3(nd), dim3(TPBB), 0, stream, P, B, slot); break;
-        default: launch_pdl(bz_kernel<0>, dim3(nd), dim3(TPBB), 0, stream, P, B, slot); break;
-        }
-        launch_pdl(bcoarse_kernel, dim3(cgrid), dim3(256), 0, stream, P, B, B.d, B.alpha, slot, 1);
-        switch (P.KS) {
-        case 1: launch_pdl(by_flat2_kernel<1>, dim3(fgrid), dim3(256), 0, stream, P, B, slot); break;
-        case 6: launch_pdl(by_flat2_kernel<6>, dim3(fgrid), dim3(256), 0, stream, P, B, slot); break;
-        default: launch_pdl(by_flat2_kernel<0>, dim3(fgrid), dim3(256), 0, stream, P, B, slot); break;
-        }
+        with_kwidth(P.KS, [&](auto kc) {
+            constexpr int KC = decltype(kc)::value;
+            const int c = KC ? blk.cluster : 1;
+            launch_cluster(bz_kernel<KC>, c, dim3(nd * c), dim3(256), 0, stream, P, B, slot);
+            launch_pdl(bcoarse_kernel, dim3(cgrid), dim3(256), 0, stream, P, B, B.d, B.alpha, slot, 1);
+            launch_pdl(byp_flat2_kernel<KC>, dim3(fgrid), dim3(256), 0, stream, P, B, slot);
+        });
+    } else {
+        launch_pdl(bp_kernel, dim3(fgrid), dim3(256), 0, stream, P, B, slot);
     }
-    launch_pdl(bp_kernel, dim3(blk.flat_grid), dim3(256), 0, stream, P, B, slot);
     if (mixed) launch_symm(Flow, true, nullptr, B.p32, B.Ap, slot, 1);
     else launch_symm(F64, false, B.p, nullptr, B.Ap, slot, 1);
     launch_block_hybrid(B.p, B.Ap, slot, 1, B.scal + SC_PAP * blk.nr);
-    switch (P.KS) {
-    case 1: launch_pdl(bupdate_kernel<1>, dim3(nd), dim3(TPBB), 0, stream, P, B, slot); break;
-    case 6: launch_pdl(bupdate_kernel<6>, dim3(nd), dim3(TPBB), 0, stream, P, B, slot); break;
-    default: launch_pdl(bupdate_kernel<0>, dim3(nd), dim3(TPBB), 0, stream, P, B, slot); break;
-    }
+    with_kwidth(P.KS, [&](auto kc) {
+        constexpr int KC = decltype(kc)::value;
+        const int c = KC ? blk.cluster : 1;
+        launch_cluster(bupdate_kernel<KC>, c, dim3(nd * c), dim3(256), 0, stream, P, B, slot);
+    });
 }
 
 // panels of the mixed blocks for the asynchronous tensor-core SYMM (built before any graph capture)
