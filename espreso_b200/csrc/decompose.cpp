@@ -4,7 +4,6 @@
 #include <algorithm>
 #include <array>
 #include <numeric>
-#include <unordered_map>
 
 #include "common.h"
 
@@ -119,25 +118,25 @@ Decomposition decompose(const ElementData &el, int ndomains_hint, const std::vec
             for (int i = 0; i < 4; ++i) k[i] = en[kHexFaces[f][i]];
             std::sort(k, k + 4);
         };
-        int k[4];
-        for (size_t e = 0; e < ne; ++e) {
-            if (el.node_ptr[e + 1] - el.node_ptr[e] != 8) continue;
+        // sorted nodes of every face; first node -1 for elements without the HEXA8 faces
+        std::vector<std::array<int, 4>> key(6 * ne);
+#pragma omp parallel for schedule(static)
+        for (long long e = 0; e < (long long)ne; ++e) {
+            const bool hex = el.node_ptr[e + 1] - el.node_ptr[e] == 8;
             for (int f = 0; f < 6; ++f) {
-                face_key(e, f, k);
-                cnt[k[0] + 1]++;
+                int k[4] = {-1, -1, -1, -1};
+                if (hex) face_key((size_t)e, f, k);
+                key[6 * (size_t)e + f] = {k[0], k[1], k[2], k[3]};
             }
         }
+        for (const auto &k : key)
+            if (k[0] >= 0) cnt[k[0] + 1]++;
         for (int n = 0; n < dec.n_nodes; ++n) cnt[n + 1] += cnt[n];
         std::vector<std::array<int, 3>> rest(cnt[dec.n_nodes]);   // the other three nodes of each face
         {
             std::vector<int> fill(cnt.begin(), cnt.end() - 1);
-            for (size_t e = 0; e < ne; ++e) {
-                if (el.node_ptr[e + 1] - el.node_ptr[e] != 8) continue;
-                for (int f = 0; f < 6; ++f) {
-                    face_key(e, f, k);
-                    rest[fill[k[0]]++] = {k[1], k[2], k[3]};
-                }
-            }
+            for (const auto &k : key)
+                if (k[0] >= 0) rest[fill[k[0]]++] = {k[1], k[2], k[3]};
         }
         std::vector<char> extf(rest.size(), 0);
 #pragma omp parallel for schedule(dynamic, 1024)
@@ -176,10 +175,21 @@ Decomposition decompose(const ElementData &el, int ndomains_hint, const std::vec
         if (ga != gb) return ga < gb ? -1 : 1;
         return 0;
     };
-    std::sort(used.begin(), used.end(), [&](int a, int b) {
-        int c = cmp_key(a, b);
-        return c != 0 ? c < 0 : a < b;
-    });
+    {
+        // the first domain of the list is the leading key: nodes bucketed by it, buckets sorted in parallel
+        std::vector<int> cnt(dec.ndom + 1, 0), sorted(used.size());
+        for (int n : used) cnt[dlist[dptr[n]] + 1]++;
+        for (int d = 0; d < dec.ndom; ++d) cnt[d + 1] += cnt[d];
+        std::vector<int> fill(cnt.begin(), cnt.end() - 1);
+        for (int n : used) sorted[fill[dlist[dptr[n]]]++] = n;
+        used.swap(sorted);
+#pragma omp parallel for schedule(dynamic, 1)
+        for (int d = 0; d < dec.ndom; ++d)
+            std::sort(used.begin() + cnt[d], used.begin() + cnt[d + 1], [&](int a, int b) {
+                int c = cmp_key(a, b);
+                return c != 0 ? c < 0 : a < b;
+            });
+    }
     dec.node_order = used;
     dec.interval_ptr.push_back(0);
     for (size_t i = 1; i <= used.size(); ++i)
@@ -198,15 +208,20 @@ Decomposition decompose(const ElementData &el, int ndomains_hint, const std::vec
 
     FETI_LOG(3, "FETI4I: decompose t_order %.3f s\n", now_s() - tdec);
     // domain local node numbering (interval by interval)
-    dec.g2l.assign(dec.ndom, std::unordered_map<int, int>());
+    dec.g2l.assign(dec.ndom, NodeMap());
+    // the intervals of every domain, ascending, with the domain's position in the interval's list
+    std::vector<std::vector<std::pair<int, int>>> dom_int(dec.ndom);
     for (int p = 0; p < nint; ++p)
-        for (int d : dec.interval_domains[p])
-            for (int i = dec.interval_ptr[p]; i < dec.interval_ptr[p + 1]; ++i) {
-                int node = used[i];
-                dec.g2l[d][node] = (int)dec.dom[d].nodes.size();
-                dec.dom[d].nodes.push_back(node);
-            }
-    for (int d = 0; d < dec.ndom; ++d) dec.dom[d].ndofs = dpn * (int)dec.dom[d].nodes.size();
+        for (int k = 0; k < (int)dec.interval_domains[p].size(); ++k) dom_int[dec.interval_domains[p][k]].emplace_back(p, k);
+#pragma omp parallel for schedule(dynamic, 1)
+    for (int d = 0; d < dec.ndom; ++d) {
+        DomainRows &D = dec.dom[d];
+        for (auto &pk : dom_int[d])
+            D.nodes.insert(D.nodes.end(), used.begin() + dec.interval_ptr[pk.first], used.begin() + dec.interval_ptr[pk.first + 1]);
+        dec.g2l[d].reserve(D.nodes.size());
+        for (size_t i = 0; i < D.nodes.size(); ++i) dec.g2l[d][D.nodes[i]] = (int)i;
+        D.ndofs = dpn * (int)D.nodes.size();
+    }
 
     FETI_LOG(3, "FETI4I: decompose t_g2l %.3f s\n", now_s() - tdec);
     // Dirichlet nodes per (component, interval); values by (node, comp)
@@ -243,12 +258,24 @@ Decomposition decompose(const ElementData &el, int ndomains_hint, const std::vec
     dec.n_lambda = (int)off;
 
     auto pair_index = [](int a, int b, int m) { return a * m - a * (a + 1) / 2 + (b - a - 1); };
-    for (int p = 0; p < nint; ++p) {
-        const std::vector<int> &doms = dec.interval_domains[p];
-        int m = (int)doms.size();
-        for (int k = 0; k < m; ++k) {
-            DomainRows &D = dec.dom[doms[k]];
-            const auto &g2l = dec.g2l[doms[k]];
+    // rows of every domain: per interval the Dirichlet rows, then the gluing rows
+#pragma omp parallel for schedule(dynamic, 1)
+    for (int d = 0; d < dec.ndom; ++d) {
+        DomainRows &D = dec.dom[d];
+        const NodeMap &g2l = dec.g2l[d];
+        auto row = [&](int64_t lam, int node, int c, double sign, int other, double value) {
+            D.lam.push_back((int)lam);
+            D.dof.push_back(dpn * g2l.at(node) + c);
+            D.sign.push_back(sign);
+            D.c.push_back(value);
+            D.other.push_back(other);
+            D.node.push_back(node);
+            D.comp.push_back(c);
+        };
+        for (auto &pk : dom_int[d]) {
+            const int p = pk.first, k = pk.second;
+            const std::vector<int> &doms = dec.interval_domains[p];
+            const int m = (int)doms.size();
             // Dirichlet rows (redundant: every domain of the interval)
             int64_t lm = 0;
             for (int c = 0; c < dpn; ++c) {
@@ -256,51 +283,30 @@ Decomposition decompose(const ElementData &el, int ndomains_hint, const std::vec
                 int64_t base = doff[p] + (int64_t)k * cnt + lm;
                 int t = 0;
                 for (int i = dec.interval_ptr[p]; i < dec.interval_ptr[p + 1]; ++i) {
-                    int node = used[i];
-                    size_t key = (size_t)node * dpn + c;
-                    if (!dmask[key]) continue;
-                    D.lam.push_back((int)(base + t++));
-                    D.dof.push_back(dpn * g2l.at(node) + c);
-                    D.sign.push_back(1.0);
-                    D.c.push_back(dval[key]);
-                    D.other.push_back(-1);
-                    D.node.push_back(node);
-                    D.comp.push_back(c);
+                    const size_t key = (size_t)used[i] * dpn + c;
+                    if (dmask[key]) row(base + t++, used[i], c, 1.0, -1, dval[key]);
                 }
                 lm += (int64_t)m * cnt;
             }
-        }
-        if (m > 1) {
-            int npairs = m * (m - 1) / 2;
-            for (int k = 0; k < m; ++k) {
-                DomainRows &D = dec.dom[doms[k]];
-                const auto &g2l = dec.g2l[doms[k]];
-                int64_t counter = 0;
-                for (int c = 0; c < dpn; ++c)
-                    for (int i = dec.interval_ptr[p]; i < dec.interval_ptr[p + 1]; ++i) {
-                        int node = used[i];
-                        if (dmask[(size_t)node * dpn + c]) continue;
-                        int64_t base = goff[p] + counter * npairs;
-                        for (int a = 0; a < k; ++a) {
-                            D.lam.push_back((int)(base + pair_index(a, k, m)));
-                            D.sign.push_back(-1.0);
-                            D.other.push_back(doms[a]);
-                            D.dof.push_back(dpn * g2l.at(node) + c); D.c.push_back(0.0); D.node.push_back(node); D.comp.push_back(c);
-                        }
-                        for (int b = k + 1; b < m; ++b) {
-                            D.lam.push_back((int)(base + pair_index(k, b, m)));
-                            D.sign.push_back(1.0);
-                            D.other.push_back(doms[b]);
-                            D.dof.push_back(dpn * g2l.at(node) + c); D.c.push_back(0.0); D.node.push_back(node); D.comp.push_back(c);
-                        }
-                        ++counter;
-                    }
-            }
+            if (m < 2) continue;
+            const int npairs = m * (m - 1) / 2;
+            int64_t counter = 0;
+            for (int c = 0; c < dpn; ++c)
+                for (int i = dec.interval_ptr[p]; i < dec.interval_ptr[p + 1]; ++i) {
+                    const int node = used[i];
+                    if (dmask[(size_t)node * dpn + c]) continue;
+                    const int64_t base = goff[p] + counter * npairs;
+                    for (int a = 0; a < k; ++a) row(base + pair_index(a, k, m), node, c, -1.0, doms[a], 0.0);
+                    for (int b = k + 1; b < m; ++b) row(base + pair_index(k, b, m), node, c, 1.0, doms[b], 0.0);
+                    ++counter;
+                }
         }
     }
     FETI_LOG(3, "FETI4I: decompose t_rows %.3f s\n", now_s() - tdec);
     // rows in ascending multiplier order
-    for (auto &D : dec.dom) {
+#pragma omp parallel for schedule(dynamic, 1)
+    for (int d = 0; d < dec.ndom; ++d) {
+        DomainRows &D = dec.dom[d];
         size_t n = D.lam.size();
         std::vector<size_t> ord(n);
         std::iota(ord.begin(), ord.end(), 0);
@@ -317,6 +323,7 @@ Decomposition decompose(const ElementData &el, int ndomains_hint, const std::vec
 
 void compute_weights(Decomposition &dec, const std::vector<std::vector<double>> *diags) {
     const int dpn = dec.dpn;
+#pragma omp parallel for schedule(dynamic, 1)
     for (int d = 0; d < dec.ndom; ++d) {
         DomainRows &D = dec.dom[d];
         for (size_t i = 0; i < D.lam.size(); ++i) {
@@ -338,7 +345,7 @@ void restrict_subdomains(Decomposition &dec, int first, int count) {
                "FETI4I: the owned subdomain range [" + std::to_string(first) + ", " + std::to_string(first + count) +
                    ") is outside the " + std::to_string(dec.ndom) + " subdomains");
     dec.dom = std::vector<DomainRows>(dec.dom.begin() + first, dec.dom.begin() + first + count);
-    dec.g2l = std::vector<std::unordered_map<int, int>>(dec.g2l.begin() + first, dec.g2l.begin() + first + count);
+    dec.g2l = std::vector<NodeMap>(dec.g2l.begin() + first, dec.g2l.begin() + first + count);
     dec.ndom = count;
 }
 

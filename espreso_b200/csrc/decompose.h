@@ -8,10 +8,71 @@
 #pragma once
 
 #include <cstdint>
-#include <unordered_map>
+#include <memory>
+#include <new>
+#include <stdexcept>
+#include <utility>
 #include <vector>
 
 namespace feti {
+
+// Vector storage that resize() leaves uninitialised: large arrays are written by all host threads, which
+// also touch their pages first.
+template <typename T>
+struct UninitAllocator : std::allocator<T> {
+    template <typename U>
+    struct rebind {
+        using other = UninitAllocator<U>;
+    };
+    template <typename U>
+    void construct(U *p) { ::new ((void *)p) U; }
+    template <typename U, typename... A>
+    void construct(U *p, A &&...a) { ::new ((void *)p) U(std::forward<A>(a)...); }
+};
+
+// int -> int map of one subdomain's nodes: open addressing in one array.  Every host pass over the
+// elements looks up each of their nodes; chained hash maps made those look-ups, and the copies of the
+// decomposition, most of the host time of a new instance.
+class NodeMap {
+public:
+    void reserve(size_t n) {
+        size_t cap = 16;
+        while (cap < 2 * n) cap *= 2;
+        if (cap > slots.size()) rehash(cap);
+    }
+    int &operator[](int key) {
+        if (2 * (count + 1) > slots.size()) rehash(slots.empty() ? 16 : 2 * slots.size());
+        std::pair<int, int> &s = slots[find(key)];
+        if (s.first < 0) {
+            s = {key, 0};
+            ++count;
+        }
+        return s.second;
+    }
+    int at(int key) const {
+        if (!slots.empty() && key >= 0) {
+            const std::pair<int, int> &s = slots[find(key)];
+            if (s.first == key) return s.second;
+        }
+        throw std::out_of_range("FETI4I: a node is not part of the subdomain");
+    }
+
+private:
+    std::vector<std::pair<int, int>> slots;   // key -1: empty (nodes are not negative)
+    size_t count = 0;
+    size_t find(int key) const {
+        const size_t mask = slots.size() - 1;
+        size_t i = (size_t)((unsigned)key * 0x9E3779B1u >> 4) & mask;
+        while (slots[i].first >= 0 && slots[i].first != key) i = (i + 1) & mask;
+        return i;
+    }
+    void rehash(size_t cap) {
+        std::vector<std::pair<int, int>> old(cap, std::pair<int, int>(-1, 0));
+        old.swap(slots);
+        for (const auto &s : old)
+            if (s.first >= 0) slots[find(s.first)] = s;
+    }
+};
 
 struct ElementData {
     int type = 0;        // FETI4IMatrixType
@@ -19,7 +80,7 @@ struct ElementData {
     std::vector<int> etype;
     std::vector<int64_t> node_ptr, dof_ptr, val_ptr;
     std::vector<int> nodes, dofs;     // already shifted by index_base
-    std::vector<double> vals;         // row-major dofsSize^2 per element
+    std::vector<double, UninitAllocator<double>> vals;   // row-major dofsSize^2 per element
     std::vector<int> partition;       // element -> subdomain (optional)
     std::vector<int> sub_cluster;     // subdomain -> cluster for Hybrid Total FETI (optional)
     size_t nelem() const { return etype.size(); }
@@ -50,7 +111,7 @@ struct Decomposition {
     std::vector<int> node_ndom;       // number of domains sharing each node
     std::vector<int> node_interval;   // node -> interval index
     std::vector<DomainRows> dom;
-    std::vector<std::unordered_map<int, int>> g2l;  // per domain: global node -> local node
+    std::vector<NodeMap> g2l;  // per domain: global node -> local node
 };
 
 // Build the numbering.  `dirichlet` holds caller DOFs (already shifted) and values.

@@ -29,12 +29,18 @@ void clear_last_error() { t_last_error.clear(); }
 
 using namespace feti;
 
+// Element data is shared by a matrix and the instances made from it (the reference copies it,
+// wrapper.cpp:156-162): whoever changes it while others hold it takes its own copy first.
 struct FETI4IStructMatrix {
-    ElementData el;
+    std::shared_ptr<ElementData> el = std::make_shared<ElementData>();
+    ElementData &own() {
+        if (el.use_count() > 1) el = std::make_shared<ElementData>(*el);
+        return *el;
+    }
 };
 
 struct FETI4IStructInstance {
-    ElementData el;              // copy of the element data (the reference copies too, wrapper.cpp:156-162)
+    std::shared_ptr<ElementData> el;
     std::vector<double> rhs;
     std::vector<int> l2g;
     std::vector<int> dir_idx;
@@ -113,6 +119,46 @@ void add_element(ElementData &el, int type, int nn, const FETI4IInt *nodes, int 
     el.val_ptr.push_back((int64_t)el.vals.size());
 }
 
+// The same for a block of elements on all host threads; false, with nothing added, when an element is
+// to be skipped or an index does not fit (the caller then adds them one by one).
+bool add_elements(ElementData &el, int type, long long ne, int nn, const FETI4IInt *nodes, int nd, const FETI4IInt *dofs,
+                  const double *values) {
+    if (ne == 0) return true;
+    const FETI4IInt base = el.index_base;
+    auto fits = [base](FETI4IInt v) {
+        return (FETI4IInt)(v - base) >= (FETI4IInt)INT32_MIN && (FETI4IInt)(v - base) <= (FETI4IInt)INT32_MAX;
+    };
+    int plain = 1;
+#pragma omp parallel for schedule(static) reduction(&& : plain)
+    for (long long e = 0; e < ne; ++e) {
+        bool zero = true, ok = true;
+        for (int i = 0; i < nd && zero; ++i) zero = values[(size_t)e * nd * nd + i] == 0.0;
+        for (int i = 0; i < nn; ++i) ok = ok && fits(nodes[(size_t)e * nn + i]);
+        for (int i = 0; i < nd; ++i) ok = ok && fits(dofs[(size_t)e * nd + i]);
+        plain = plain && !zero && ok;
+    }
+    if (!plain) return false;
+    if (el.node_ptr.empty()) { el.node_ptr.push_back(0); el.dof_ptr.push_back(0); el.val_ptr.push_back(0); }
+    const size_t e0 = el.etype.size(), n0 = el.nodes.size(), d0 = el.dofs.size(), v0 = el.vals.size();
+    el.etype.resize(e0 + ne, type);
+    el.nodes.resize(n0 + (size_t)ne * nn);
+    el.dofs.resize(d0 + (size_t)ne * nd);
+    el.vals.resize(v0 + (size_t)ne * nd * nd);
+    el.node_ptr.resize(e0 + ne + 1);
+    el.dof_ptr.resize(e0 + ne + 1);
+    el.val_ptr.resize(e0 + ne + 1);
+#pragma omp parallel for schedule(static)
+    for (long long e = 0; e < ne; ++e) {
+        for (int i = 0; i < nn; ++i) el.nodes[n0 + (size_t)e * nn + i] = (int)(nodes[(size_t)e * nn + i] - base);
+        for (int i = 0; i < nd; ++i) el.dofs[d0 + (size_t)e * nd + i] = (int)(dofs[(size_t)e * nd + i] - base);
+        std::memcpy(el.vals.data() + v0 + (size_t)e * nd * nd, values + (size_t)e * nd * nd, sizeof(double) * (size_t)nd * nd);
+        el.node_ptr[e0 + e + 1] = (int64_t)(n0 + (size_t)(e + 1) * nn);
+        el.dof_ptr[e0 + e + 1] = (int64_t)(d0 + (size_t)(e + 1) * nd);
+        el.val_ptr[e0 + e + 1] = (int64_t)(v0 + (size_t)(e + 1) * nd * nd);
+    }
+    return true;
+}
+
 // The decomposition depends on the element structure, the partition and the Dirichlet DOFs only;
 // a matrix update with the same structure keeps it.
 bool same_structure(const ElementData &a, const ElementData &b) {
@@ -120,7 +166,9 @@ bool same_structure(const ElementData &a, const ElementData &b) {
            a.dofs == b.dofs && a.partition == b.partition && a.index_base == b.index_base;
 }
 
-void build(FETI4IStructInstance *I, bool keep_decomposition = false) {
+// keep_tuning: the tile sizes and options are those of the instance's last build, so are the SYMV variant and
+// the work items that were timed then.
+void build(FETI4IStructInstance *I, bool keep_decomposition = false, bool keep_tuning = false) {
     const int *io = I->iopt;
     g_verbose = io[FETI4I_VERBOSE_LEVEL];
     FETI_CHECK(io[FETI4I_FETI_METHOD] == 0 || io[FETI4I_FETI_METHOD] == 1,
@@ -133,17 +181,17 @@ void build(FETI4IStructInstance *I, bool keep_decomposition = false) {
     FETI_CHECK(io[FETI4I_MAX_ITERATIONS] > 0, "FETI4I: MAX_ITERATIONS must be positive");
     double t0 = now_s();
     if (!keep_decomposition) {
-        I->dec_full = decompose(I->el, io[FETI4I_SUBDOMAINS], I->dir_idx, I->dir_val);
+        I->dec_full = decompose(*I->el, io[FETI4I_SUBDOMAINS], I->dir_idx, I->dir_val);
         FETI_LOG(2, "FETI4I: decomposition %.3f s\n", now_s() - t0);
     }
     I->dec = I->dec_full;   // preprocess keeps the owned subdomains of a partitioned problem
     PrepOptions po;
     po.method = io[FETI4I_FETI_METHOD];
-    if (po.method == 1 && !I->el.sub_cluster.empty()) {
-        FETI_CHECK((int)I->el.sub_cluster.size() == I->dec.ndom,
-                   "FETI4I: the cluster partition lists " + std::to_string(I->el.sub_cluster.size()) +
+    if (po.method == 1 && !I->el->sub_cluster.empty()) {
+        FETI_CHECK((int)I->el->sub_cluster.size() == I->dec.ndom,
+                   "FETI4I: the cluster partition lists " + std::to_string(I->el->sub_cluster.size()) +
                        " subdomains, the problem has " + std::to_string(I->dec.ndom));
-        po.sub_cluster = I->el.sub_cluster;
+        po.sub_cluster = I->el->sub_cluster;
     }
     po.precond = prec;
     po.owned_first = (int)I->ext[FETI4I_EXT_OWNED_FIRST];
@@ -158,9 +206,11 @@ void build(FETI4IStructInstance *I, bool keep_decomposition = false) {
     if (const char *b = std::getenv("FETI4I_DEVICE_PREP_BATCH_BYTES")) po.device_mem = std::strtoull(b, nullptr, 10);
     // the previous device solver (and its tile stores) goes first: a rebuild must not hold two
     // copies of the device data at once
+    TilePlans plans;
+    if (keep_tuning && I->gpu) plans = I->gpu->tile_plans();
     I->gpu.reset();
     I->prep = Prep();
-    preprocess(I->el, I->dec, I->rhs, po, I->prep);
+    preprocess(*I->el, I->dec, I->rhs, po, I->prep);
     I->t_prep = now_s() - t0;
     FETI_LOG(1, "FETI4I: %d subdomains, %d multipliers, %d kernel vectors, preprocessing %.2f s\n", I->dec.ndom,
              I->dec.n_lambda, I->prep.n_kern, I->t_prep);
@@ -184,7 +234,7 @@ void build(FETI4IStructInstance *I, bool keep_decomposition = false) {
     if (I->ext[FETI4I_EXT_HOST_ONLY] == 0.0) {
         double t1 = now_s();
         I->gpu.reset(new GpuSolver());
-        I->gpu->upload(I->dec, I->prep, so);
+        I->gpu->upload(I->dec, I->prep, so, plans);
         I->t_upload = now_s() - t1;
     }
 }
@@ -225,8 +275,8 @@ void FETI4ICreateStiffnessMatrix(FETI4IMatrix *matrix, FETI4IInt type, FETI4IInt
         FETI_CHECK(type == FETI4I_REAL_SYMMETRIC_POSITIVE_DEFINITE,
                    "FETI4I: only REAL_SYMMETRIC_POSITIVE_DEFINITE matrices are supported by the explicit-Schur solver");
         auto *m = new FETI4IStructMatrix();
-        m->el.type = (int)type;
-        m->el.index_base = narrow(indexBase, "indexBase");
+        m->el->type = (int)type;
+        m->el->index_base = narrow(indexBase, "indexBase");
         g_matrices.push_back(m);
         *matrix = m;
     });
@@ -237,7 +287,7 @@ void FETI4IAddElement(FETI4IMatrix matrix, FETI4IInt type, FETI4IInt nodesSize, 
     guarded([&] {
         auto *m = check_matrix(matrix);
         FETI_CHECK(nodesSize > 0 && dofsSize > 0 && nodes && dofs && values, "FETI4I: invalid element data");
-        add_element(m->el, (int)type, narrow(nodesSize, "nodesSize"), nodes, narrow(dofsSize, "dofsSize"), dofs,
+        add_element(m->own(), (int)type, narrow(nodesSize, "nodesSize"), nodes, narrow(dofsSize, "dofsSize"), dofs,
                     values);
     });
 }
@@ -247,11 +297,13 @@ void FETI4IAddElements(FETI4IMatrix matrix, FETI4IInt type, FETI4IInt nelems, FE
     guarded([&] {
         auto *m = check_matrix(matrix);
         FETI_CHECK(nelems >= 0 && nodesSize > 0 && dofsSize > 0 && nodes && dofs && values, "FETI4I: invalid element data");
-        m->el.etype.reserve(m->el.etype.size() + nelems);
-        m->el.vals.reserve(m->el.vals.size() + (size_t)nelems * dofsSize * dofsSize);
         const int nn = narrow(nodesSize, "nodesSize"), nd = narrow(dofsSize, "dofsSize");
+        ElementData &el = m->own();
+        if (add_elements(el, (int)type, (long long)nelems, nn, nodes, nd, dofs, values)) return;
+        el.etype.reserve(el.etype.size() + nelems);
+        el.vals.reserve(el.vals.size() + (size_t)nelems * dofsSize * dofsSize);
         for (FETI4IInt e = 0; e < nelems; ++e)
-            add_element(m->el, (int)type, nn, nodes + (size_t)e * nn, nd, dofs + (size_t)e * nd,
+            add_element(el, (int)type, nn, nodes + (size_t)e * nn, nd, dofs + (size_t)e * nd,
                         values + (size_t)e * nd * nd);
     });
 }
@@ -259,8 +311,8 @@ void FETI4IAddElements(FETI4IMatrix matrix, FETI4IInt type, FETI4IInt nelems, FE
 void FETI4ISetSubdomainPartition(FETI4IMatrix matrix, FETI4IInt size, FETI4IInt *elem2sub) {
     guarded([&] {
         auto *m = check_matrix(matrix);
-        FETI_CHECK(size == (FETI4IInt)m->el.nelem(), "FETI4I: partition size differs from the number of added elements");
-        m->el.partition = narrow_all(elem2sub, (size_t)size, "a subdomain index");
+        FETI_CHECK(size == (FETI4IInt)m->el->nelem(), "FETI4I: partition size differs from the number of added elements");
+        m->own().partition = narrow_all(elem2sub, (size_t)size, "a subdomain index");
     });
 }
 
@@ -268,7 +320,7 @@ void FETI4ISetClusterPartition(FETI4IMatrix matrix, FETI4IInt nsubdomains, const
     guarded([&] {
         auto *m = check_matrix(matrix);
         FETI_CHECK(nsubdomains >= 0 && (nsubdomains == 0 || sub2cluster), "FETI4I: invalid cluster partition");
-        m->el.sub_cluster = narrow_all(sub2cluster, (size_t)nsubdomains, "a cluster index");
+        m->own().sub_cluster = narrow_all(sub2cluster, (size_t)nsubdomains, "a cluster index");
     });
 }
 
@@ -315,7 +367,7 @@ void FETI4ICreateInstance(FETI4IInstance *instance, FETI4IMatrix matrix, FETI4II
         I->rhs.assign(rhs, rhs + size);
         if (l2g) I->l2g = narrow_all(l2g, (size_t)size, "an l2g entry");
         for (FETI4IInt i = 0; i < dirichlet_size; ++i) {
-            I->dir_idx.push_back(narrow(dirichlet_indices[i] - m->el.index_base, "a Dirichlet index"));
+            I->dir_idx.push_back(narrow(dirichlet_indices[i] - m->el->index_base, "a Dirichlet index"));
             I->dir_val.push_back(dirichlet_values[i]);
         }
         for (int k = 0; k < FETI4I_INTEGER_OPTIONS_SIZE; ++k) I->iopt[k] = narrow(integer_options[k], "an option");
@@ -438,12 +490,15 @@ void FETI4IUpdateStiffnessMatrix(FETI4IInstance instance, FETI4IMatrix stiffness
     guarded([&] {
         auto *I = check_instance(instance);
         auto *m = check_matrix(stiffnessMatrix);
-        std::vector<int> part = I->el.partition;
-        ElementData el = m->el;
-        if (el.partition.empty() && part.size() == el.nelem()) el.partition = part;
-        const bool keep = same_structure(el, I->el);
-        I->el = std::move(el);
-        build(I, keep);
+        std::shared_ptr<ElementData> el = m->el;
+        const std::vector<int> &part = I->el->partition;
+        if (el->partition.empty() && part.size() == el->nelem()) {
+            el = std::make_shared<ElementData>(*el);
+            el->partition = part;
+        }
+        const bool keep = same_structure(*el, *I->el);
+        I->el = el;
+        build(I, keep, keep);
     });
 }
 
@@ -452,33 +507,38 @@ void FETI4IUpdateStiffnessMatrixScaled(FETI4IInstance instance, FETI4IMatrix sti
     guarded([&] {
         auto *I = check_instance(instance);
         auto *m = check_matrix(stiffnessMatrix);
-        const ElementData &src = m->el;
+        const std::shared_ptr<ElementData> held = m->el;
+        const ElementData &src = *held;
         FETI_CHECK(size == (FETI4IInt)src.nelem() && (size == 0 || scale),
                    "FETI4I: one scale per stored element of the matrix is required");
-        std::vector<int> part = I->el.partition;
-        const bool keep = same_structure(src, I->el) ||
-                          (src.partition.empty() && part.size() == src.nelem() && [&] {
-                              ElementData probe;
-                              probe.etype = src.etype; probe.node_ptr = src.node_ptr; probe.dof_ptr = src.dof_ptr;
-                              probe.nodes = src.nodes; probe.dofs = src.dofs; probe.partition = part;
-                              probe.index_base = src.index_base;
-                              return same_structure(probe, I->el);
-                          }());
+        // the matrix's structure, or with no partition of its own the instance's partition on it
+        const bool borrow = src.partition.empty() && I->el->partition.size() == src.nelem();
+        bool keep = same_structure(src, *I->el);
+        if (!keep && borrow) {
+            const ElementData &o = *I->el;
+            keep = src.etype == o.etype && src.node_ptr == o.node_ptr && src.dof_ptr == o.dof_ptr && src.nodes == o.nodes &&
+                   src.dofs == o.dofs && src.index_base == o.index_base;
+        }
+        // the instance's element data: its own, or a copy of the structure where others hold it
+        if (!keep || I->el.use_count() > 1) {
+            const ElementData &from = keep ? *I->el : src;
+            auto el = std::make_shared<ElementData>();
+            el->type = from.type; el->index_base = from.index_base; el->etype = from.etype;
+            el->node_ptr = from.node_ptr; el->dof_ptr = from.dof_ptr; el->val_ptr = from.val_ptr;
+            el->nodes = from.nodes; el->dofs = from.dofs; el->sub_cluster = from.sub_cluster;
+            el->partition = !keep && borrow ? I->el->partition : from.partition;
+            I->el = el;
+        }
         // K_e := scale_e * K_e of the matrix object (element after element, in parallel)
-        I->el.vals.resize(src.vals.size());
+        ElementData &dst = *I->el;
+        dst.vals.resize(src.vals.size());
         const long long ne = (long long)src.nelem();
 #pragma omp parallel for schedule(static)
         for (long long e = 0; e < ne; ++e) {
             const double s_ = scale[e];
-            for (int64_t k = src.val_ptr[e]; k < src.val_ptr[e + 1]; ++k) I->el.vals[k] = s_ * src.vals[k];
+            for (int64_t k = src.val_ptr[e]; k < src.val_ptr[e + 1]; ++k) dst.vals[k] = s_ * src.vals[k];
         }
-        if (!keep) {
-            std::vector<double> v = std::move(I->el.vals);
-            I->el = src;
-            I->el.vals = std::move(v);
-            if (I->el.partition.empty() && part.size() == I->el.nelem()) I->el.partition = part;
-        }
-        build(I, keep);
+        build(I, keep, keep);
     });
 }
 
@@ -487,18 +547,7 @@ void FETI4IUpdateRhs(FETI4IInstance instance, FETI4IInt size, FETI4IReal *values
         auto *I = check_instance(instance);
         FETI_CHECK(size >= 0 && (size == 0 || values), "FETI4I: invalid right-hand side");
         I->rhs.assign(values, values + size);
-        // subdomain loads: value / multiplicity (src/assembler/physics/precomputed.cpp:61-65)
-        const int dpn = I->dec.dpn;
-        for (int d = 0; d < I->dec.ndom; ++d) {
-            SubPrep &S = I->prep.sub[d];
-            const DomainRows &D = I->dec.dom[d];
-            for (int a = 0; a < (int)D.nodes.size(); ++a)
-                for (int c = 0; c < dpn; ++c) {
-                    int dof = I->dec.node_dof[(size_t)D.nodes[a] * dpn + c];
-                    double v = (dof >= 0 && dof < (int)I->rhs.size()) ? I->rhs[dof] : 0.0;
-                    S.f[dpn * a + c] = v / I->dec.node_ndom[D.nodes[a]];
-                }
-        }
+        subdomain_loads(I->dec, I->rhs, I->prep);
         I->rhs_on_device = false;
     });
 }
@@ -509,7 +558,7 @@ void FETI4IUpdateDirichlet(FETI4IInstance instance, FETI4IInt size, FETI4IInt *i
         std::vector<int> idx;
         std::vector<double> val;
         for (FETI4IInt i = 0; i < size; ++i) {
-            idx.push_back(narrow(indices[i] - I->el.index_base, "a Dirichlet index"));
+            idx.push_back(narrow(indices[i] - I->el->index_base, "a Dirichlet index"));
             val.push_back(values[i]);
         }
         std::vector<int> a = idx, b = I->dir_idx;
@@ -562,7 +611,7 @@ void FETI4IGetStats(FETI4IInstance instance, FETI4IInt size, FETI4IReal *stats) 
         v[FETI4I_STAT_DEVICE_BYTES] = I->gpu ? (double)I->gpu->device_bytes() : 0.0;
         v[FETI4I_STAT_FINAL_NORM] = I->stats.final_norm;
         v[FETI4I_STAT_TOLERANCE] = I->stats.tol;
-        v[FETI4I_STAT_ELEMENTS] = (double)I->el.nelem();
+        v[FETI4I_STAT_ELEMENTS] = (double)I->el->nelem();
         v[FETI4I_STAT_PREP_DEVICE_MS] = I->prep.t_device_factor_ms;
         v[FETI4I_STAT_PREP_DEVICE_FLOPS] = I->prep.device_factor_flops;
         v[FETI4I_STAT_KPLUS_TILES] = I->gpu ? I->gpu->kplus_tile_fraction() : 0.0;
@@ -732,7 +781,7 @@ void FETI4IElementEnergies(FETI4IInstance instance, FETI4IInt size, const FETI4I
         auto *I = check_instance(instance);
         FETI_CHECK(I->gpu, "FETI4I: no device solver");
         FETI_CHECK(size > 0 && u && v && out, "FETI4I: invalid vectors");
-        I->gpu->element_energies(I->el, u, v, size, out);
+        I->gpu->element_energies(*I->el, u, v, size, out);
     });
 }
 

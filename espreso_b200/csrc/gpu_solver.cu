@@ -3142,7 +3142,17 @@ bool cuda_available(std::string &why) {
     return true;
 }
 
-void GpuSolver::upload(const Decomposition &dec, const Prep &prep, const SolveOptions &opt) {
+TilePlans GpuSolver::tile_plans() const {
+    const Impl &I = *impl;
+    TilePlans p;
+    if (!I.opt.autotune) return p;
+    p.f64 = {I.F64.kernel, I.F64.class_tpi};
+    p.low = {I.Flow.kernel, I.Flow.class_tpi};
+    p.dir = {I.Dir.kernel, I.Dir.class_tpi};
+    return p;
+}
+
+void GpuSolver::upload(const Decomposition &dec, const Prep &prep, const SolveOptions &opt, const TilePlans &plans) {
     const double tu0 = now_s();
     Impl &I = *impl;
     I.opt = opt;
@@ -3190,10 +3200,11 @@ void GpuSolver::upload(const Decomposition &dec, const Prep &prep, const SolveOp
     std::vector<int> partner(NL, -1), tidx(NL), rkof(NL), rnk(NL);
     std::vector<double> ws(NL), minv(NL), Gl((size_t)NL * KS, 0.0);
     I.max_ni = 0;
+    for (int d = 0; d < nd; ++d) I.max_ni = std::max(I.max_ni, prep.sub[d].ni);
+#pragma omp parallel for schedule(dynamic, 1)
     for (int d = 0; d < nd; ++d) {
         const DomainRows &D = dec.dom[d];
         const SubPrep &S = prep.sub[d];
-        I.max_ni = std::max(I.max_ni, S.ni);
         for (int r = 0; r < S.ni; ++r) {
             int e = loff[d] + r;
             int l = D.lam[r];
@@ -3213,6 +3224,7 @@ void GpuSolver::upload(const Decomposition &dec, const Prep &prep, const SolveOp
     // partner data of every row (shortens the dependent-load chains of the assembly)
     std::vector<int> ptidx(NL, -1), pkof(NL, 0), pnk(NL, 0);
     std::vector<double> pws(NL, 0.0), Gp((size_t)NL * KS, 0.0);
+#pragma omp parallel for schedule(static)
     for (int e = 0; e < NL; ++e) {
         int q = partner[e];
         if (q < 0) continue;
@@ -3231,33 +3243,42 @@ void GpuSolver::upload(const Decomposition &dec, const Prep &prep, const SolveOp
         for (int e = 0; e < NL; ++e) trow_idx[fill[tidx[e]]++] = e;
     }
     // lumped preconditioner: K_TT of each subdomain in sliced ELL (32 rows, column-major)
-    std::vector<int> slice0(nd + 1, 0), ell_ptr, ell_w;
-    std::vector<unsigned short> ell_col;
-    std::vector<double> ell_val;
+    std::vector<int> slice0(nd + 1, 0);
     I.max_nt = 0;
     for (int d = 0; d < nd; ++d) {
         const SubPrep &S = prep.sub[d];
         I.max_nt = std::max(I.max_nt, S.t);
-        slice0[d + 1] = slice0[d];
-        if (opt.precond != PREC_LUMPED) continue;
-        FETI_CHECK(S.t < 65536, "FETI4I: too many interface DOFs in one subdomain for the lumped kernel");
-        for (int t0 = 0; t0 < S.t; t0 += 32) {
-            int w = 0;
-            for (int t = t0; t < std::min(S.t, t0 + 32); ++t) w = std::max(w, S.KT_ptr[t + 1] - S.KT_ptr[t]);
-            ell_ptr.push_back((int)ell_val.size());
-            ell_w.push_back(w);
-            size_t base = ell_val.size();
-            ell_val.resize(base + (size_t)32 * w, 0.0);
-            ell_col.resize(base + (size_t)32 * w, 0);
+        FETI_CHECK(opt.precond != PREC_LUMPED || S.t < 65536,
+                   "FETI4I: too many interface DOFs in one subdomain for the lumped kernel");
+        slice0[d + 1] = slice0[d] + (opt.precond == PREC_LUMPED ? (S.t + 31) / 32 : 0);
+    }
+    std::vector<int> ell_ptr(slice0[nd]), ell_w(slice0[nd], 0);
+#pragma omp parallel for schedule(dynamic, 1)
+    for (int d = 0; d < nd; ++d)
+        for (int sl = slice0[d]; sl < slice0[d + 1]; ++sl) {
+            const SubPrep &S = prep.sub[d];
+            const int t0 = 32 * (sl - slice0[d]);
+            for (int t = t0; t < std::min(S.t, t0 + 32); ++t) ell_w[sl] = std::max(ell_w[sl], S.KT_ptr[t + 1] - S.KT_ptr[t]);
+        }
+    size_t ell_n = 0;
+    for (int sl = 0; sl < slice0[nd]; ++sl) {
+        ell_ptr[sl] = (int)ell_n;
+        ell_n += (size_t)32 * ell_w[sl];
+    }
+    std::vector<unsigned short> ell_col(ell_n, 0);
+    std::vector<double> ell_val(ell_n, 0.0);
+#pragma omp parallel for schedule(dynamic, 1)
+    for (int d = 0; d < nd; ++d)
+        for (int sl = slice0[d]; sl < slice0[d + 1]; ++sl) {
+            const SubPrep &S = prep.sub[d];
+            const int t0 = 32 * (sl - slice0[d]);
             for (int t = t0; t < std::min(S.t, t0 + 32); ++t)
                 for (int j = S.KT_ptr[t]; j < S.KT_ptr[t + 1]; ++j) {
-                    size_t o = base + (size_t)(j - S.KT_ptr[t]) * 32 + (t - t0);
+                    const size_t o = (size_t)ell_ptr[sl] + (size_t)(j - S.KT_ptr[t]) * 32 + (t - t0);
                     ell_val[o] = S.KT_val[j];
                     ell_col[o] = (unsigned short)S.KT_col[j];
                 }
-            slice0[d + 1]++;
         }
-    }
     std::vector<int> tbase(NT), tslot(NT);
     for (int d = 0; d < nd; ++d)
         for (int t = toff[d]; t < toff[d + 1]; ++t) {
@@ -3376,12 +3397,21 @@ void GpuSolver::upload(const Decomposition &dec, const Prep &prep, const SolveOp
         I.build_tiles(I.Dir, SCHUR_FP64, dm, dn, dv, opt.tiles_per_item, d64);
     }
     if (opt.autotune) {
+        auto tune = [&](TileSetHost &T, const TilePlan &plan, double *x, double *y, int n) {
+            if ((int)plan.class_tpi.size() == kSizeClasses) {
+                T.kernel = plan.kernel;
+                T.class_tpi = plan.class_tpi;
+                I.itemize(T, T.class_tpi, -1);
+            } else {
+                I.autotune(T, x, y, n);
+            }
+        };
         CUDA_CHECK(cudaMemset(P.w, 0, sizeof(double) * NL));
-        if (!I.implicit) I.autotune(I.F64, P.w, I.Ax64, NL);
-        if (opt.schur_precision != SCHUR_FP64) I.autotune(I.Flow, P.w, I.Ax64, NL);
+        if (!I.implicit) tune(I.F64, plans.f64, P.w, I.Ax64, NL);
+        if (opt.schur_precision != SCHUR_FP64) tune(I.Flow, plans.low, P.w, I.Ax64, NL);
         if (opt.precond == PREC_DIRICHLET) {
             CUDA_CHECK(cudaMemset(P.uT, 0, sizeof(double) * NT));
-            I.autotune(I.Dir, P.uT, P.vT, NT);
+            tune(I.Dir, plans.dir, P.uT, P.vT, NT);
         }
     }
     const double tu2 = now_s();
@@ -4158,7 +4188,8 @@ void GpuSolver::element_energies(const ElementData &el, const double *u, const d
         FETI_CHECK(el.dof_ptr[e + 1] - el.dof_ptr[e] == nd, "FETI4I: element energies need elements of one size");
     if (I.el_dofs == nullptr || I.el_count != ne || I.el_nd != nd) {
         I.el_dofs = I.upload(el.dofs);
-        I.el_K = I.upload(el.vals);
+        I.el_K = I.alloc<double>(std::max<size_t>(el.vals.size(), 1));
+        CUDA_CHECK(cudaMemcpyAsync(I.el_K, el.vals.data(), sizeof(double) * el.vals.size(), cudaMemcpyHostToDevice, I.stream));
         I.el_out = I.alloc<double>(ne);
         I.el_count = ne;
         I.el_nd = nd;

@@ -45,11 +45,22 @@ struct SolveStats {
     bool converged = false;
 };
 
+// What the SYMV autotuner chose for the FP64, low-precision and Dirichlet tiles (empty: nothing yet).
+struct TilePlan {
+    int kernel = 0;
+    std::vector<int> class_tpi;
+};
+struct TilePlans {
+    TilePlan f64, low, dir;
+};
+
 class GpuSolver {
 public:
     GpuSolver();
     ~GpuSolver();
-    void upload(const Decomposition &dec, const Prep &prep, const SolveOptions &opt);
+    // plans: of an earlier upload of the same sizes and options, used instead of timing the variants again
+    void upload(const Decomposition &dec, const Prep &prep, const SolveOptions &opt, const TilePlans &plans = TilePlans());
+    TilePlans tile_plans() const;
     // Dual PCG on device-resident b (lambda space), e (kernel space); outputs lambda and alpha.
     void set_rhs(const std::vector<double> &b, const std::vector<double> &e);
     void solve(SolveStats &st);

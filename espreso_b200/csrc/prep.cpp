@@ -543,12 +543,28 @@ static void prep_all_device(const ElementData &el, const Decomposition &dec, con
              t1 - t0, t2 - t1, dt.device_ms, dt.flops * 1e-9, dt.batches, now_s() - t2);
 }
 
+void subdomain_loads(const Decomposition &dec, const std::vector<double> &rhs, Prep &out) {
+    const int dpn = dec.dpn;
+#pragma omp parallel for schedule(dynamic, 1)
+    for (int d = 0; d < dec.ndom; ++d) {
+        SubPrep &S = out.sub[d];
+        const DomainRows &D = dec.dom[d];
+        for (int a = 0; a < (int)D.nodes.size(); ++a)
+            for (int c = 0; c < dpn; ++c) {
+                int dof = dec.node_dof[(size_t)D.nodes[a] * dpn + c];
+                double v = (dof >= 0 && dof < (int)rhs.size()) ? rhs[dof] : 0.0;
+                S.f[dpn * a + c] = v / dec.node_ndom[D.nodes[a]];
+            }
+    }
+}
+
 void preprocess(const ElementData &el, Decomposition &dec, const std::vector<double> &rhs, const PrepOptions &opt,
                 Prep &out) {
     const int dpn = dec.dpn;
     double t0 = now_s();
     // K diagonals for the B1 scaling (diagonal of each subdomain matrix)
     std::vector<std::vector<double>> diags(dec.ndom);
+#pragma omp parallel for schedule(dynamic, 1)
     for (int d = 0; d < dec.ndom; ++d) {
         diags[d].assign(dec.dom[d].ndofs, 0.0);
         for (int e : dec.dom[d].elems) {
@@ -605,17 +621,7 @@ void preprocess(const ElementData &el, Decomposition &dec, const std::vector<dou
     for (int d = 0; d < dec.ndom; ++d)
         if (!errors[d].empty()) throw Error(errors[d] + " (subdomain " + std::to_string(d) + ")");
 
-    // subdomain right-hand sides: caller DOF value divided by its multiplicity
-    for (int d = 0; d < dec.ndom; ++d) {
-        SubPrep &S = out.sub[d];
-        const DomainRows &D = dec.dom[d];
-        for (int a = 0; a < (int)D.nodes.size(); ++a)
-            for (int c = 0; c < dpn; ++c) {
-                int dof = dec.node_dof[(size_t)D.nodes[a] * dpn + c];
-                double v = (dof >= 0 && dof < (int)rhs.size()) ? rhs[dof] : 0.0;
-                S.f[dpn * a + c] = v / dec.node_ndom[D.nodes[a]];
-            }
-    }
+    subdomain_loads(dec, rhs, out);
     out.t_factor = now_s() - t0;
     FETI_LOG(2, "FETI4I: subdomain preprocessing %.3f s\n", out.t_factor);
 

@@ -102,6 +102,10 @@ struct PrepOptions {
     int owned_first = 0, owned_count = 0;   // partitioned dual problem: prepare these subdomains only (count 0: all)
 };
 
+// Subdomain loads f_i: the caller's DOF values divided by their multiplicity
+// (src/assembler/physics/precomputed.cpp:61-65).
+void subdomain_loads(const Decomposition &dec, const std::vector<double> &rhs, Prep &out);
+
 // rhs: caller DOF vector (size >= max DOF + 1); split per subdomain by multiplicity.
 void preprocess(const ElementData &el, Decomposition &dec, const std::vector<double> &rhs, const PrepOptions &opt,
                 Prep &out);

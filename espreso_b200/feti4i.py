@@ -241,7 +241,7 @@ class Instance:
         self.n = n
 
     def solve(self, out=None):
-        sol = np.zeros(self.n) if out is None else out
+        sol = np.empty(self.n) if out is None else out   # the library writes every entry
         self.lib.FETI4ISolve(self.h, sol.size, _dp(sol))
         _check(self.lib)
         return sol
@@ -249,7 +249,7 @@ class Instance:
     def solve_multi(self, rhs):
         """rhs (nrhs, size) -> solutions (nrhs, size), solved together."""
         R = np.ascontiguousarray(np.atleast_2d(rhs), dtype=np.float64)
-        out = np.zeros_like(R)
+        out = np.empty_like(R)   # the library writes every entry
         self.lib.FETI4ISolveMulti(self.h, R.shape[0], R.shape[1], _dp(R), _dp(out))
         _check(self.lib)
         return out
