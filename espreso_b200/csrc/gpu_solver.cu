@@ -1027,40 +1027,53 @@ __global__ void tol_kernel(DevProblem P) {
 }
 
 // w = r - G^T alpha (||w||^2 total), u_T = B^T (W w) and, for the lumped preconditioner, v_T = K_TT u_T
-// (sliced ELL).  With no preconditioner y = w and rho = y.w is taken here.  One cluster per subdomain:
-// its CTAs share the rows, then the touched DOFs (slice sl belongs to rank sl mod C), and exchange w and
-// u_T through distributed shared memory.  A slice's entries are dealt to `parts` warps, eight loads in
-// flight each: one warp over a row of up to 81 entries was the longest chain of the kernel.
+// (sliced ELL).  With no preconditioner y = w and rho = y.w is taken here.
+// CL: a cluster of CTAs per subdomain; its CTAs share the rows, then the touched DOFs (slice sl belongs to
+// rank sl mod C), and exchange w and u_T through distributed shared memory.  Otherwise one CTA of 512
+// threads, three per SM: with the cluster code (54 registers) only two fitted, and 512 subdomains took
+// 45 us instead of 30 (cold caches).  A slice's entries go to `parts` warps where a CTA has fewer slices
+// than warps: a row has up to 81 entries.
 constexpr int ELL_PARTS = 4;
-template <int PRECOND, int KC>
-__global__ void __launch_bounds__(TPB1) w_prec_kernel(DevProblem P, int slot, int parts) {
+template <int PRECOND, int KC, bool CL>
+__global__ void __launch_bounds__(CL ? TPB1 / 2 : TPB1, CL ? 5 : 3) w_prec_kernel(DevProblem P, int slot, int parts) {
     pdl_enter();
     extern __shared__ double sm[];
     __shared__ double sh[32];
     const int iter = P.st->iter_base + slot;
     if (skip_iter(P.st, iter)) return;
-    cluster_enter();
-    const int C = (int)cluster_size_x(), rank = (int)cluster_rank_x(), dsub = blockIdx.x / C;
+    if (CL) cluster_enter();
+    const int C = CL ? (int)cluster_size_x() : 1, rank = CL ? (int)cluster_rank_x() : 0, dsub = blockIdx.x / C;
     const int e0 = P.loff[dsub], ni = P.loff[dsub + 1] - e0;
     const int t0 = P.toff[dsub], nt = P.toff[dsub + 1] - t0;
     double *wsm = sm;          // w of the subdomain rows
     double *u = sm + ni;       // B^T W w on the touched DOFs
     double *acc = u + nt;      // parts x (32 x slices of this rank)
+    auto publish = [&](double *q, double v) {   // to the same place in every CTA of the cluster
+        if (CL)
+            for (int r = 0; r < C; ++r) st_cluster(q, (unsigned)r, v);
+        else
+            *q = v;
+    };
+    auto barrier = [&] {
+        if (CL) {
+            cluster_arrive();
+            cluster_wait();
+        } else {
+            __syncthreads();
+        }
+    };
     double ww = 0.0;
-    cluster_entered();
+    if (CL) cluster_entered();
     for (int i = rank * blockDim.x + threadIdx.x; i < ni; i += C * blockDim.x) {
         const int e = e0 + i;
         const double wv = __ldg(P.r + e) - gt_alpha_k<KC>(P, e, P.alpha);
         P.w[e] = wv;
         if (PRECOND == PREC_NONE) P.y[e] = wv;
-        else if (C == 1) wsm[i] = wv;
-        else
-            for (int q = 0; q < C; ++q) st_cluster(wsm + i, (unsigned)q, wv);
+        else publish(wsm + i, wv);
         ww += wv * wv * __ldg(P.minv + e);
     }
     if (PRECOND != PREC_NONE) {
-        cluster_arrive();
-        cluster_wait();
+        barrier();
         const int nsl = (nt + 31) / 32, mine = nsl > rank ? (nsl - rank + C - 1) / C : 0;
         for (int q = threadIdx.x; q < 32 * mine; q += blockDim.x) {
             const int t = 32 * (rank + (q >> 5) * C) + (q & 31);
@@ -1070,15 +1083,12 @@ __global__ void __launch_bounds__(TPB1) w_prec_kernel(DevProblem P, int slot, in
                 const int e = __ldg(P.trow_idx + j);
                 s += __ldg(P.ws + e) * wsm[e - e0];
             }
-            if (PRECOND != PREC_LUMPED) P.uT[t0 + t] = s;
-            else if (C == 1) u[t] = s;
-            else
-                for (int r = 0; r < C; ++r) st_cluster(u + t, (unsigned)r, s);
+            if (PRECOND == PREC_LUMPED) publish(u + t, s);
+            else P.uT[t0 + t] = s;
             if (PRECOND == PREC_WEIGHT) P.vT[t0 + t] = s;
         }
         if (PRECOND == PREC_LUMPED) {
-            cluster_arrive();
-            cluster_wait();
+            barrier();
             const int lane = threadIdx.x & 31, nw = blockDim.x >> 5, sl0 = P.slice0[dsub];
             for (int q = threadIdx.x >> 5; q < mine * parts; q += nw) {
                 const int k = q / parts, pt = q - k * parts, sl = sl0 + rank + k * C;
@@ -1086,31 +1096,34 @@ __global__ void __launch_bounds__(TPB1) w_prec_kernel(DevProblem P, int slot, in
                 const int j0 = wd * pt / parts, j1 = wd * (pt + 1) / parts;
                 const int base = __ldg(P.ell_ptr + sl) + lane;
                 double s0 = 0.0, s1 = 0.0;
-                int j = j0;
-                for (; j + 8 <= j1; j += 8) {
-                    double v[8];
-                    int c[8];
+                constexpr int FL = CL ? 8 : 4;   // entries in flight
+                for (int j = j0; j < j1; j += FL) {
+                    double v[FL];
+                    int c[FL];
 #pragma unroll
-                    for (int x = 0; x < 8; ++x) {
-                        v[x] = __ldg(P.ell_val + base + (j + x) * 32);
-                        c[x] = __ldg(P.ell_col + base + (j + x) * 32);
+                    for (int x = 0; x < FL; ++x) {
+                        const bool in = j + x < j1;
+                        v[x] = in ? __ldg(P.ell_val + base + (j + x) * 32) : 0.0;
+                        c[x] = in ? __ldg(P.ell_col + base + (j + x) * 32) : 0;
                     }
 #pragma unroll
-                    for (int x = 0; x < 8; x += 2) {
+                    for (int x = 0; x < FL; x += 2) {
                         s0 += v[x] * u[c[x]];
                         s1 += v[x + 1] * u[c[x + 1]];
                     }
                 }
-#pragma unroll 4
-                for (; j < j1; ++j) s0 += __ldg(P.ell_val + base + j * 32) * u[__ldg(P.ell_col + base + j * 32)];
-                acc[(pt * mine + k) * 32 + lane] = s0 + s1;
+                const int t = 32 * (rank + k * C) + lane;
+                if (parts > 1) acc[(pt * mine + k) * 32 + lane] = s0 + s1;
+                else if (t < nt) P.vT[t0 + t] = s0 + s1;
             }
-            __syncthreads();
-            for (int q = threadIdx.x; q < 32 * mine; q += blockDim.x) {
-                const int t = 32 * (rank + (q >> 5) * C) + (q & 31);
-                double s = 0.0;
-                for (int pt = 0; pt < parts; ++pt) s += acc[pt * mine * 32 + q];
-                if (t < nt) P.vT[t0 + t] = s;
+            if (parts > 1) {
+                __syncthreads();
+                for (int q = threadIdx.x; q < 32 * mine; q += blockDim.x) {
+                    const int t = 32 * (rank + (q >> 5) * C) + (q & 31);
+                    double s = 0.0;
+                    for (int pt = 0; pt < parts; ++pt) s += acc[pt * mine * 32 + q];
+                    if (t < nt) P.vT[t0 + t] = s;
+                }
             }
         }
     }
@@ -2956,9 +2969,13 @@ static void set_smem_limits() {
     set_tile_limits<SCHUR_BF16>(v);
     auto w_limits = [&](auto kc) {
         constexpr int KC = decltype(kc)::value;
-        CUDA_CHECK(cudaFuncSetAttribute(w_prec_kernel<PREC_LUMPED, KC>, cudaFuncAttributeMaxDynamicSharedMemorySize, v));
-        CUDA_CHECK(cudaFuncSetAttribute(w_prec_kernel<PREC_WEIGHT, KC>, cudaFuncAttributeMaxDynamicSharedMemorySize, v));
-        CUDA_CHECK(cudaFuncSetAttribute(w_prec_kernel<PREC_DIRICHLET, KC>, cudaFuncAttributeMaxDynamicSharedMemorySize, v));
+        auto one = [&](auto kernel) { CUDA_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, v)); };
+        one(w_prec_kernel<PREC_LUMPED, KC, true>);
+        one(w_prec_kernel<PREC_WEIGHT, KC, true>);
+        one(w_prec_kernel<PREC_DIRICHLET, KC, true>);
+        one(w_prec_kernel<PREC_LUMPED, KC, false>);
+        one(w_prec_kernel<PREC_WEIGHT, KC, false>);
+        one(w_prec_kernel<PREC_DIRICHLET, KC, false>);
     };
     w_limits(std::integral_constant<int, 0>());
     w_limits(std::integral_constant<int, 1>());
@@ -2995,12 +3012,18 @@ void GpuSolver::Impl::launch_iteration(int slot, bool with_replacement) {
     const dim3 vgrid(P.nd * vec_cluster);
     with_kwidth(P.KS, [&](auto kc) {
         constexpr int KC = decltype(kc)::value;
-        auto w_prec = opt.precond == PREC_NONE     ? w_prec_kernel<PREC_NONE, KC>
-                      : opt.precond == PREC_LUMPED ? w_prec_kernel<PREC_LUMPED, KC>
-                      : opt.precond == PREC_WEIGHT ? w_prec_kernel<PREC_WEIGHT, KC>
-                                                   : w_prec_kernel<PREC_DIRICHLET, KC>;
-        launch_cluster(w_prec, vec_cluster, vgrid, dim3(vec_cluster > 1 ? TPB1 / 2 : TPB1),
-                       opt.precond == PREC_NONE ? 0 : w_smem, stream, P, slot, ell_parts);
+        auto pick = [&](auto cl) {
+            constexpr bool CL = decltype(cl)::value;
+            return opt.precond == PREC_NONE     ? w_prec_kernel<PREC_NONE, KC, CL>
+                   : opt.precond == PREC_LUMPED ? w_prec_kernel<PREC_LUMPED, KC, CL>
+                   : opt.precond == PREC_WEIGHT ? w_prec_kernel<PREC_WEIGHT, KC, CL>
+                                                : w_prec_kernel<PREC_DIRICHLET, KC, CL>;
+        };
+        const size_t wsm = opt.precond == PREC_NONE ? 0 : w_smem;
+        if (vec_cluster > 1)
+            launch_cluster(pick(std::true_type()), vec_cluster, vgrid, dim3(TPB1 / 2), wsm, stream, P, slot, ell_parts);
+        else
+            launch_pdl(pick(std::false_type()), vgrid, dim3(TPB1), wsm, stream, P, slot, ell_parts);
     });
     if (opt.precond != PREC_NONE) {
         if (opt.precond == PREC_DIRICHLET) {
@@ -3288,8 +3311,9 @@ void GpuSolver::upload(const Decomposition &dec, const Prep &prep, const SolveOp
     {
         const int slices = ((I.max_nt + 31) / 32 + I.vec_cluster - 1) / I.vec_cluster;
         auto bytes = [&](int parts) { return sizeof(double) * (size_t)(I.max_ni + I.max_nt + 32 * parts * slices); };
-        I.ell_parts = ELL_PARTS;
-        while (I.ell_parts > 1 && bytes(I.ell_parts) > 200 * 1024) I.ell_parts /= 2;
+        const int warps = (I.vec_cluster > 1 ? TPB1 / 2 : TPB1) / 32;
+        I.ell_parts = std::max(1, std::min(ELL_PARTS, (warps + slices - 1) / std::max(1, slices)));
+        while (I.ell_parts > 1 && bytes(I.ell_parts) > 200 * 1024) --I.ell_parts;
         I.w_smem = bytes(I.ell_parts);
     }
     FETI_CHECK(sizeof(double) * (size_t)(I.max_nt + I.max_ni) <= 200 * 1024,
