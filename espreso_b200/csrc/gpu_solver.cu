@@ -5077,9 +5077,15 @@ tile_symm_kernel(TileSetDev ts, DevProblem P, BlockDev B, const double *x64, con
     if (s_last) {
         if (mode == 1) {
             __threadfence();
+            __shared__ double s_dot[256];
+            double t = 0.0;
+            for (int q = threadIdx.x / NR; q < nunits; q += 256 / NR)
+                t += __ldcg(&B.unit_dot[(size_t)q * NR + threadIdx.x % NR]);
+            s_dot[threadIdx.x] = t;
+            __syncthreads();
             if (threadIdx.x < NR) {
-                double t = 0.0;
-                for (int q = 0; q < nunits; ++q) t += __ldcg(&B.unit_dot[(size_t)q * NR + threadIdx.x]);
+                t = 0.0;
+                for (int g = 0; g < 256 / NR; ++g) t += s_dot[g * NR + threadIdx.x];
                 B.scal[SC_PAP * NR + threadIdx.x] = t;
             }
         }
@@ -5097,8 +5103,12 @@ tile_symm_kernel(TileSetDev ts, DevProblem P, BlockDev B, const double *x64, con
 // (I, J) for J >= I and the transpose of the stored tile (J, I) for J < I, read straight from
 // global memory in fragment order (every 32-byte sector once), as 4 x NR/8 blocks of 8 x 8 over
 // 8 k-steps of 4.  x rows past the subdomain read as zero.
+// Sixteen warps per SM at 8 and 16 columns (128 registers): a warp waits for one tile at a time, and 64
+// subdomains have fewer tile rows than two waves of eight.  With this and the dots summed by all threads
+// of the last CTA, not by one warp, 64 subdomains of 6^3 elasticity elements and 16 columns take 121 us
+// instead of 141.
 template <int NR>
-__global__ void __launch_bounds__(256, 1)
+__global__ void __launch_bounds__(256, NR == 32 ? 1 : 2)
 tile_symm_mma_kernel(TileSetDev ts, DevProblem P, BlockDev B, const double *x64, double *out, const int2 *units,
                      int nunits, int slot, int mode) {
     pdl_enter();
@@ -5190,9 +5200,16 @@ tile_symm_mma_kernel(TileSetDev ts, DevProblem P, BlockDev B, const double *x64,
     if (s_last) {
         if (mode == 1) {
             __threadfence();
+            // p.Ap of every column from the units' dots, all threads, in a fixed order
+            __shared__ double s_dot[256];
+            double t = 0.0;
+            for (int q = threadIdx.x / NR; q < nunits; q += 256 / NR)
+                t += __ldcg(&B.unit_dot[(size_t)q * NR + threadIdx.x % NR]);
+            s_dot[threadIdx.x] = t;
+            __syncthreads();
             if (threadIdx.x < NR) {
-                double t = 0.0;
-                for (int q = 0; q < nunits; ++q) t += __ldcg(&B.unit_dot[(size_t)q * NR + threadIdx.x]);
+                t = 0.0;
+                for (int g = 0; g < 256 / NR; ++g) t += s_dot[g * NR + threadIdx.x];
                 B.scal[SC_PAP * NR + threadIdx.x] = t;
             }
         }
@@ -5476,10 +5493,16 @@ tile_symm_tc_kernel(TileSetDev ts, DevProblem P, BlockDev B, const float *x32, d
     if (s_last) {
         if (mode == 1) {
             __threadfence();
-            if (tid < NR) {
-                double t = 0.0;
-                for (int q = 0; q < nunits; ++q) t += __ldcg(&B.unit_dot[(size_t)q * NR + tid]);
-                B.scal[SC_PAP * NR + tid] = t;
+            __shared__ double s_dot[256];
+            double t = 0.0;
+            for (int q = threadIdx.x / NR; q < nunits; q += 256 / NR)
+                t += __ldcg(&B.unit_dot[(size_t)q * NR + threadIdx.x % NR]);
+            s_dot[threadIdx.x] = t;
+            __syncthreads();
+            if (threadIdx.x < NR) {
+                t = 0.0;
+                for (int g = 0; g < 256 / NR; ++g) t += s_dot[g * NR + threadIdx.x];
+                B.scal[SC_PAP * NR + threadIdx.x] = t;
             }
         }
         if (tid == 0) {
