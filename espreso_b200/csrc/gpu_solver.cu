@@ -1401,13 +1401,14 @@ __device__ __forceinline__ long long ltile(int T, int I, int J) {
 // to every CTA of the cluster, and the target blocks t > s are dealt to the warps of the whole cluster
 // (warp t mod NW), each block to one warp for the whole sweep: its partial sums need no atomics and no
 // barrier.  The warp that owns block s + 1 applies its tile first, solves the diagonal block (staged by
-// cp.async since its previous turn) and publishes it while the others still work on step s; every other
+// cp.async some steps before) and publishes it while the others still work on step s; every other
 // warp has arrived at the cluster barrier of step s + 1 before its own tiles, so the barrier costs the
 // publishing warp's path only.  Every CTA keeps the whole vector in shared memory.
 // Per pass, one CTA per subdomain before / clusters now: 64 subdomains of 8^3 elasticity elements (0.64 GB
-// of nonzero tiles) 905 / 255 us, 64 uneven ones of up to 7,560 DOFs (largest 0.14 GB) 5.2 / 1.5 ms, 27
-// of 6^3 271 / 100 us; 512 of 10^3 heat elements fill the chip either way (592 us, clusters of one).
+// of nonzero tiles) 905 / 255 us, 64 uneven ones of up to 7,560 DOFs (largest 0.14 GB) 5.2 / 0.95 ms, 27
+// of 6^3 271 / 87 us; 512 of 10^3 heat elements fill the chip either way (592 us, clusters of one).
 constexpr int KP_WARPS = 8;
+constexpr int KP_STAGES = 4;   // staged diagonal tiles per CTA
 
 struct KpTile {
     uint4 u[16];
@@ -1444,7 +1445,7 @@ __device__ __forceinline__ double kp_apply(F chunk, const double *x, int lane) {
 
 // FWD: v[32 lo ..) := L^-1 v over the blocks lo .. T-1; else v := L^-T v, blocks T-1 down to lo.  v is
 // whole and the same in every CTA on entry (after a cluster barrier) and on return.
-// dbuf: 8 KB per warp, or null (the diagonal tiles are then read when they are needed).
+// dbuf: KP_STAGES tiles, or null (the diagonal tiles are then read when they are needed).
 template <bool FWD>
 __device__ void kp_sweep(const uint4 *tiles, const unsigned *mask, int mw, int T, int lo, double *v, uint4 *dbuf) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -1455,10 +1456,13 @@ __device__ void kp_sweep(const uint4 *tiles, const unsigned *mask, int mw, int T
         const int a = blk(s), b = blk(t);
         return tiles + (size_t)(FWD ? ltile(T, b, a) : ltile(T, a, b)) * (TILE * 16);
     };
-    uint4 *mydiag = dbuf ? dbuf + warp * (TILE * 16) : nullptr;
+    // diagonal tiles are staged 2 C steps ahead by the warp that will use them; a CTA owns every C-th step,
+    // and the buffer of step s was last read at step s - KP_STAGES C, which is published by then
+    auto buffer = [&](int s) { return dbuf ? dbuf + ((s / C) % KP_STAGES) * (TILE * 16) : nullptr; };
     auto stage_diag = [&](int s) {
-        if (!mydiag || s >= steps) return;
+        if (!dbuf || s >= steps) return;
         const uint4 *src = tile(s, s);
+        uint4 *mydiag = buffer(s);
 #pragma unroll
         for (int q = 0; q < 16; ++q)
             asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((unsigned)__cvta_generic_to_shared(mydiag + q * 32 + lane)),
@@ -1468,18 +1472,16 @@ __device__ void kp_sweep(const uint4 *tiles, const unsigned *mask, int mw, int T
     };
     // solve the diagonal block of step s from this CTA's finished v and publish it (one warp)
     auto publish = [&](int s) {
-        const uint4 *dp = mydiag ? mydiag : tile(s, s);
+        const uint4 *dp = dbuf ? buffer(s) : tile(s, s);
         asm volatile("cp.async.wait_group 0;" ::: "memory");   // each lane reads what it copied itself
         double *vb = v + TILE * blk(s);
         __syncwarp();
         const double y = kp_apply<FWD>([&](int q) { return dp[q * 32 + lane]; }, vb, lane);
         __syncwarp();
         for (int r = 0; r < C; ++r) st_cluster(vb + idx, (unsigned)r, y);
-        __syncwarp();
-        stage_diag(s + NW);
     };
     if (steps <= 0) return;   // the same for the whole cluster
-    stage_diag(W);
+    if (W <= 2 * C) stage_diag(W);
     if (W == 0) publish(0);
     cluster_arrive();
     for (int s = 0; s < steps; ++s) {
@@ -1492,6 +1494,7 @@ __device__ void kp_sweep(const uint4 *tiles, const unsigned *mask, int mw, int T
         KpTile a;
         if (t < steps && (!crit || t == s + 1)) kp_load(a, tile(s, t), lane);
         cluster_wait();                                   // block s is solved in every CTA
+        if (s > 0 && W == (s + 2 * C) % NW) stage_diag(s + 2 * C);
         const double *x = v + TILE * blk(s);
         if (crit) {
             if (t == s + 1) {
@@ -1529,7 +1532,7 @@ __device__ __forceinline__ uint4 *kp_dbuf(double *v, KpSmem sm) {
 __device__ const unsigned *kp_mask(const KplusDev &K, int d, double *v, KpSmem sm) {
     const unsigned *g = K.mask + K.moff[d];
     if (!(sm.parts & KPS_MASK)) return g;
-    unsigned *m = reinterpret_cast<unsigned *>(v + (size_t)TILE * sm.vblocks + (sm.parts & KPS_DIAG ? KP_WARPS * TILE * TILE : 0));
+    unsigned *m = reinterpret_cast<unsigned *>(v + (size_t)TILE * sm.vblocks + (sm.parts & KPS_DIAG ? KP_STAGES * TILE * TILE : 0));
     for (int i = threadIdx.x; i < K.tn[d] * K.mw[d]; i += blockDim.x) m[i] = __ldg(g + i);
     return m;
 }
@@ -2495,7 +2498,7 @@ void GpuSolver::Impl::upload_kplus(const Decomposition &dec, const Prep &prep, c
         while (kp_cluster < 8 && max_T >= 16 * kp_cluster &&
                (2 * kp_cluster * nd <= 2 * nsm || wmax * nsm > wsum * kp_cluster))
             kp_cluster *= 2;
-        const size_t vb = sizeof(double) * TILE * (size_t)max_T, db = sizeof(double) * KP_WARPS * TILE * TILE,
+        const size_t vb = sizeof(double) * TILE * (size_t)max_T, db = sizeof(double) * KP_STAGES * TILE * TILE,
                      mb = sizeof(unsigned) * (size_t)mask_max;
         kp_smem.vblocks = max_T;
         kp_smem.parts = 0;
