@@ -2054,17 +2054,18 @@ __global__ void hyb_kz_kernel(DevProblem P, HybDev H, const int *doff, const int
         for (int k = 0; k < nk; ++k) H.z[z0 + m0 + k] = -acc[k];
 }
 
-// step 2: g_i = x_i - B0_i^T lambda0 (one thread walks a subdomain's corner entries: a corner DOF
-// can appear in several rows of one subdomain)
+// step 2: g_i = x_i - B0_i^T lambda0 (one warp per subdomain; atomics, as a corner DOF can appear in
+// several rows of one subdomain)
 __global__ void hyb_copy_kernel(const double *x, double *g, int ntot) {
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < ntot; i += gridDim.x * blockDim.x) g[i] = x[i];
 }
 __global__ void hyb_kb0_kernel(DevProblem P, HybDev H, const int *doff, double *g) {
-    const int d = blockIdx.x * blockDim.x + threadIdx.x;
+    const int d = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     if (d >= P.nd) return;
     const int z0 = H.zof[d], m0 = H.m0[d];
     const double *wc = H.w + H.cof[H.sub_cl[d]];
-    for (int j = 0; j < m0; ++j) g[doff[d] + H.b0dof[z0 + j]] -= H.b0sign[z0 + j] * wc[H.vmap[z0 + j]];
+    for (int j = threadIdx.x & 31; j < m0; j += 32)
+        atomicAdd(&g[doff[d] + H.b0dof[z0 + j]], -H.b0sign[z0 + j] * wc[H.vmap[z0 + j]]);
 }
 
 // step 3: out_i += R_i alpha_i
@@ -2658,7 +2659,7 @@ void GpuSolver::Impl::launch_kplus_dual_multi(const double *in, double *out, int
         hyb_kz_kernel<<<P.nd, 256, 0, stream>>>(P, H, d_doff, d_rofs, d_R, outj, inj);
         hyb_m_kernel<<<dim3(H.ncl, hyb_rows1), 256, sizeof(double) * H.max_nc, stream>>>(P, H, 0, 0, nullptr);
         hyb_copy_kernel<<<std::max(1, std::min(4096, (ntot + 255) / 256)), 256, 0, stream>>>(inj, hj, ntot);
-        hyb_kb0_kernel<<<(P.nd + 127) / 128, 128, 0, stream>>>(P, H, d_doff, hj);
+        hyb_kb0_kernel<<<(P.nd + 3) / 4, 128, 0, stream>>>(P, H, d_doff, hj);
         CUDA_CHECK(cudaMemcpyAsync(hyb_wsave + (size_t)j * wn, H.w, sizeof(double) * wn, cudaMemcpyDeviceToDevice,
                                    stream));
     }
@@ -2677,7 +2678,7 @@ void GpuSolver::Impl::launch_kplus_dual(const double *in, double *out) {
     hyb_kz_kernel<<<P.nd, 256, 0, stream>>>(P, H, d_doff, d_rofs, d_R, out, in);
     hyb_m_kernel<<<dim3(H.ncl, hyb_rows1), 256, sizeof(double) * H.max_nc, stream>>>(P, H, 0, 0, nullptr);
     hyb_copy_kernel<<<std::max(1, std::min(4096, (ntot + 255) / 256)), 256, 0, stream>>>(in, d_h, ntot);
-    hyb_kb0_kernel<<<(P.nd + 127) / 128, 128, 0, stream>>>(P, H, d_doff, d_h);
+    hyb_kb0_kernel<<<(P.nd + 3) / 4, 128, 0, stream>>>(P, H, d_doff, d_h);
     launch_kplus(d_h, out);
     hyb_kr_kernel<<<P.nd, 256, 0, stream>>>(P, H, d_doff, d_rofs, d_R, out);
     CUDA_CHECK(cudaGetLastError());
