@@ -1,6 +1,7 @@
 // Shared helpers of the FETI4I B200 library: error state, timing, small utilities.
 #pragma once
 
+#include <exception>
 #include <chrono>
 #include <cstdint>
 #include <cstdio>
@@ -36,5 +37,22 @@ extern int g_verbose;
     do {                                                                         \
         if (::feti::g_verbose >= (level)) { std::fprintf(stderr, __VA_ARGS__); } \
     } while (0)
+
+// f(0) .. f(n - 1) on the host threads; the first exception is rethrown after the loop (none may leave an
+// OpenMP region).
+template <typename F>
+void parallel_for(int n, F &&f) {
+    std::exception_ptr error;
+#pragma omp parallel for schedule(dynamic, 1)
+    for (int i = 0; i < n; ++i) {
+        try {
+            f(i);
+        } catch (...) {
+#pragma omp critical(feti_parallel_for)
+            if (!error) error = std::current_exception();
+        }
+    }
+    if (error) std::rethrow_exception(error);
+}
 
 }  // namespace feti

@@ -213,15 +213,14 @@ Decomposition decompose(const ElementData &el, int ndomains_hint, const std::vec
     std::vector<std::vector<std::pair<int, int>>> dom_int(dec.ndom);
     for (int p = 0; p < nint; ++p)
         for (int k = 0; k < (int)dec.interval_domains[p].size(); ++k) dom_int[dec.interval_domains[p][k]].emplace_back(p, k);
-#pragma omp parallel for schedule(dynamic, 1)
-    for (int d = 0; d < dec.ndom; ++d) {
+    parallel_for(dec.ndom, [&](int d) {
         DomainRows &D = dec.dom[d];
         for (auto &pk : dom_int[d])
             D.nodes.insert(D.nodes.end(), used.begin() + dec.interval_ptr[pk.first], used.begin() + dec.interval_ptr[pk.first + 1]);
         dec.g2l[d].reserve(D.nodes.size());
         for (size_t i = 0; i < D.nodes.size(); ++i) dec.g2l[d][D.nodes[i]] = (int)i;
         D.ndofs = dpn * (int)D.nodes.size();
-    }
+    });
 
     FETI_LOG(3, "FETI4I: decompose t_g2l %.3f s\n", now_s() - tdec);
     // Dirichlet nodes per (component, interval); values by (node, comp)
@@ -259,8 +258,7 @@ Decomposition decompose(const ElementData &el, int ndomains_hint, const std::vec
 
     auto pair_index = [](int a, int b, int m) { return a * m - a * (a + 1) / 2 + (b - a - 1); };
     // rows of every domain: per interval the Dirichlet rows, then the gluing rows
-#pragma omp parallel for schedule(dynamic, 1)
-    for (int d = 0; d < dec.ndom; ++d) {
+    parallel_for(dec.ndom, [&](int d) {
         DomainRows &D = dec.dom[d];
         const NodeMap &g2l = dec.g2l[d];
         auto row = [&](int64_t lam, int node, int c, double sign, int other, double value) {
@@ -301,11 +299,10 @@ Decomposition decompose(const ElementData &el, int ndomains_hint, const std::vec
                     ++counter;
                 }
         }
-    }
+    });
     FETI_LOG(3, "FETI4I: decompose t_rows %.3f s\n", now_s() - tdec);
     // rows in ascending multiplier order
-#pragma omp parallel for schedule(dynamic, 1)
-    for (int d = 0; d < dec.ndom; ++d) {
+    parallel_for(dec.ndom, [&](int d) {
         DomainRows &D = dec.dom[d];
         size_t n = D.lam.size();
         std::vector<size_t> ord(n);
@@ -316,15 +313,14 @@ Decomposition decompose(const ElementData &el, int ndomains_hint, const std::vec
         permute_i(D.lam); permute_i(D.dof); permute_i(D.other); permute_i(D.node); permute_i(D.comp);
         permute_d(D.sign); permute_d(D.c);
         D.w.assign(n, 1.0);
-    }
+    });
     FETI_LOG(3, "FETI4I: decompose done %.3f s\n", now_s() - tdec);
     return dec;
 }
 
 void compute_weights(Decomposition &dec, const std::vector<std::vector<double>> *diags) {
     const int dpn = dec.dpn;
-#pragma omp parallel for schedule(dynamic, 1)
-    for (int d = 0; d < dec.ndom; ++d) {
+    parallel_for(dec.ndom, [&](int d) {
         DomainRows &D = dec.dom[d];
         for (size_t i = 0; i < D.lam.size(); ++i) {
             if (D.other[i] < 0) { D.w[i] = 1.0; continue; }
@@ -337,7 +333,7 @@ void compute_weights(Decomposition &dec, const std::vector<std::vector<double>> 
             double mine = (*diags)[o][dpn * dec.g2l[o].at(node) + c];
             D.w[i] = mine / tot;
         }
-    }
+    });
 }
 
 void restrict_subdomains(Decomposition &dec, int first, int count) {

@@ -564,8 +564,7 @@ void preprocess(const ElementData &el, Decomposition &dec, const std::vector<dou
     double t0 = now_s();
     // K diagonals for the B1 scaling (diagonal of each subdomain matrix)
     std::vector<std::vector<double>> diags(dec.ndom);
-#pragma omp parallel for schedule(dynamic, 1)
-    for (int d = 0; d < dec.ndom; ++d) {
+    parallel_for(dec.ndom, [&](int d) {
         diags[d].assign(dec.dom[d].ndofs, 0.0);
         for (int e : dec.dom[d].elems) {
             int nd = (int)(el.dof_ptr[e + 1] - el.dof_ptr[e]);
@@ -575,7 +574,7 @@ void preprocess(const ElementData &el, Decomposition &dec, const std::vector<dou
                 diags[d][dpn * dec.g2l[d].at(dec.dof_node[dof]) + dec.dof_comp[dof]] += Ke[(size_t)a * nd + a];
             }
         }
-    }
+    });
     compute_weights(dec, opt.scaling ? &diags : nullptr);
     // partitioned dual problem: the weights need every subdomain's diagonal; the rest only the owned block
     if (opt.owned_count > 0) {
