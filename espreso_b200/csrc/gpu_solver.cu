@@ -2215,6 +2215,7 @@ struct GpuSolver::Impl {
     void launch_symm(const TileSetHost &T, bool src32, const double *x64, const float *x32, double *out, int slot,
                      int mode);
     void launch_block_iteration(int slot);
+    void launch_br0(int replace_mode, int slot);
     // block cluster correction y -= V M V^T x for nr columns
     double *bh_z = nullptr, *bh_w = nullptr, *bh_part = nullptr;
     int *bh_done = nullptr;
@@ -4473,49 +4474,6 @@ __global__ void bgt_kernel(DevProblem P, BlockDev B, const double *a, double *xo
     if (i < P.NL * B.nr) xout[i] = gt_alpha_col(P, (i >> B.lg), (i & (B.nr - 1)), B.nr, a);
 }
 
-// r = b - assemble(Ax), d = G r, |b_j|^2 totals (initial) / replacement
-__global__ void br0_kernel(DevProblem P, BlockDev B, int replace_mode, int slot) {
-    pdl_enter();
-    __shared__ double sh[8 * 32];
-    __shared__ double cols[32];
-    if (replace_mode) {
-        const int iter = P.st->iter_base + slot;
-        if (skip_iter(P.st, iter) || P.st->replace_iter != iter) return;
-    }
-    const int nr = B.nr, dsub = blockIdx.x;
-    const int e0 = P.loff[dsub], e1 = P.loff[dsub + 1];
-    double bb = 0.0;
-    for (int i = threadIdx.x; i < (e1 - e0) * nr; i += blockDim.x) {
-        const int e = e0 + (i >> B.lg), j = (i & (nr - 1));
-        const int q = P.partner[e];
-        const size_t o = (size_t)e * nr + j;
-        const double a = B.Ax[o] + (q >= 0 ? B.Ax[(size_t)q * nr + j] : 0.0);
-        const double rv = B.bL[o] - a;
-        B.r[o] = rv;
-        bb += B.bL[o] * B.bL[o] * P.minv[e];
-    }
-    __syncthreads();
-    g_dot_cols(P, B, dsub, B.r + (size_t)e0 * nr, sh);
-    if (!replace_mode) {
-        block_sum_cols(bb, nr, sh, cols);
-        grid_total_cols(cols, B.part, B, DONE_B, B.scal + SC_BN2 * nr);
-    }
-}
-
-__global__ void bpnorm_kernel(DevProblem P, BlockDev B) {
-    __shared__ double sh[8 * 32];
-    __shared__ double cols[32];
-    const int nr = B.nr, dsub = blockIdx.x;
-    double s = 0.0;
-    for (int i = threadIdx.x; i < (P.loff[dsub + 1] - P.loff[dsub]) * nr; i += blockDim.x) {
-        const int e = P.loff[dsub] + (i >> B.lg), j = (i & (nr - 1));
-        const double u = B.r[(size_t)e * nr + j] - gt_alpha_col(P, e, j, nr, B.alpha);
-        s += u * u * P.minv[e];
-    }
-    block_sum_cols(s, nr, sh, cols);
-    grid_total_cols(cols, B.part, B, DONE_PN, B.scal + SC_PN2 * nr);
-}
-
 __global__ void btol_kernel(DevProblem P, BlockDev B) {
     const int j = threadIdx.x;
     if (j < B.nr) {
@@ -4592,6 +4550,81 @@ __device__ __forceinline__ double2 gt_alpha_colk2(const DevProblem &P, int e, in
         r.y += g[k] * x.y + gp[k] * y.y;
     }
     return r;
+}
+
+// r = b - assemble(Ax), d = G r, |b_j|^2 totals (initial) / replacement.  A cluster of CTAs per subdomain, two
+// columns per thread, as bupdate.  (One CTA of 256 threads per subdomain: 200 us for 64 subdomains and
+// 16 columns or 512 and 32.)
+template <int KC>
+__global__ void __launch_bounds__(256, 4) br0_kernel(DevProblem P, BlockDev B, int replace_mode, int slot) {
+    constexpr int NG = KC > 0 ? KC : 1;
+    pdl_enter();
+    __shared__ double sh[8 * 32];
+    __shared__ double cols[32];
+    if (replace_mode) {
+        const int iter = P.st->iter_base + slot;
+        if (skip_iter(P.st, iter) || P.st->replace_iter != iter) return;
+    }
+    cluster_enter();
+    const int C = (int)cluster_size_x(), dsub = blockIdx.x / C;
+    const int nr = B.nr, hn = nr >> 1, lh = B.lg - 1;
+    const int e0 = P.loff[dsub], e1 = P.loff[dsub + 1], cnt = (e1 - e0) * hn, jh = threadIdx.x & (hn - 1);
+    double2 gk[NG];
+#pragma unroll
+    for (int k = 0; k < NG; ++k) gk[k] = make_double2(0.0, 0.0);
+    double s0 = 0.0, s1 = 0.0;
+    const double2 *Ax = reinterpret_cast<const double2 *>(B.Ax), *bL = reinterpret_cast<const double2 *>(B.bL) + (size_t)e0 * hn;
+    double2 *r = reinterpret_cast<double2 *>(B.r) + (size_t)e0 * hn;
+#pragma unroll 2
+    for (int i = cluster_rank_x() * blockDim.x + threadIdx.x; i < cnt; i += C * blockDim.x) {
+        const int e = e0 + (i >> lh), q = __ldg(P.partner + e);
+        double2 a = __ldg(Ax + (size_t)e0 * hn + i);
+        if (q >= 0) {
+            const double2 c = __ldg(Ax + (size_t)q * hn + jh);
+            a.x += c.x;
+            a.y += c.y;
+        }
+        const double2 bv = __ldg(bL + i), rv = make_double2(bv.x - a.x, bv.y - a.y);
+        const double mv = __ldg(P.minv + e);
+        r[i] = rv;
+        s0 += bv.x * bv.x * mv;
+        s1 += bv.y * bv.y * mv;
+        if (KC > 0) {
+            const double *g = P.Gl + (size_t)e * NG;
+#pragma unroll
+            for (int k = 0; k < NG; ++k) {
+                gk[k].x += __ldg(g + k) * rv.x;
+                gk[k].y += __ldg(g + k) * rv.y;
+            }
+        }
+    }
+    if (KC > 0) {
+        g_cols_finish<NG>(P, B, dsub, gk);
+    } else {
+        __syncthreads();
+        g_dot_cols(P, B, dsub, B.r + (size_t)e0 * nr, sh);
+    }
+    if (replace_mode) return;
+    block_sum_cols2(s0, s1, nr, sh, cols);
+    grid_total_cols(cols, B.part, B, DONE_B, B.scal + SC_BN2 * nr);
+}
+
+template <int KC>
+__global__ void __launch_bounds__(256, FLAT_MIN_BLOCKS) bpnorm_kernel(DevProblem P, BlockDev B) {
+    __shared__ double sh[8 * 32];
+    __shared__ double cols[32];
+    const int nr = B.nr, lh = B.lg - 1;
+    const long long cnt = (long long)P.NL * (nr >> 1), stride = (long long)gridDim.x * blockDim.x;
+    double s0 = 0.0, s1 = 0.0;
+    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < cnt; i += stride) {
+        const int e = (int)(i >> lh), j = 2 * (int)(i & ((nr >> 1) - 1));
+        const double2 rv = __ldg(reinterpret_cast<const double2 *>(B.r) + i), ga = gt_alpha_colk2<KC>(P, e, j, nr, B.alpha);
+        const double mv = __ldg(P.minv + e);
+        s0 += (rv.x - ga.x) * (rv.x - ga.x) * mv;
+        s1 += (rv.y - ga.y) * (rv.y - ga.y) * mv;
+    }
+    block_sum_cols2(s0, s1, nr, sh, cols);
+    grid_total_cols(cols, B.part, B, DONE_PN, B.scal + SC_PN2 * nr);
 }
 
 // z = assemble(W B v_T), d = G z and rho_j = z.w, which is y.w for y = P z because w = P r lies in the range
@@ -6664,6 +6697,14 @@ void GpuSolver::Impl::launch_symm(const TileSetHost &T, bool src32, const double
     CUDA_CHECK(cudaGetLastError());
 }
 
+void GpuSolver::Impl::launch_br0(int replace_mode, int slot) {
+    with_kwidth(P.KS, [&](auto kc) {
+        constexpr int KC = decltype(kc)::value;
+        const int c = KC ? blk.cluster : 1;
+        launch_cluster(br0_kernel<KC>, c, dim3(P.nd * c), dim3(256), 0, stream, P, blk.B, replace_mode, slot);
+    });
+}
+
 void GpuSolver::Impl::launch_block_iteration(int slot) {
     const int nd = P.nd;
     const int cgrid = (P.nK + CR - 1) / CR;
@@ -6672,7 +6713,7 @@ void GpuSolver::Impl::launch_block_iteration(int slot) {
     if (mixed) {
         launch_symm(F64, false, B.x, nullptr, B.Ax, slot, 3);
         launch_block_hybrid(B.x, B.Ax, slot, 3, nullptr);
-        launch_pdl(br0_kernel, dim3(nd), dim3(TPB), 0, stream, P, B, 1, slot);
+        launch_br0(1, slot);
     }
     launch_pdl(bcoarse_kernel, dim3(cgrid), dim3(256), 0, stream, P, B, B.d, B.alpha, slot, 1);
     const int fgrid = blk.flat_grid;
@@ -6827,9 +6868,9 @@ void GpuSolver::solve_multi(const double *rhs, int nrhs, int rhs_size, double *s
     CUDA_CHECK(cudaMemsetAsync(B.p, 0, sizeof(double) * (size_t)P.NL * nr, I.stream));
     I.launch_symm(I.F64, false, B.x, nullptr, B.Ax, 0, 0);
     I.launch_block_hybrid(B.x, B.Ax, 0, 0, nullptr);
-    br0_kernel<<<nd, TPB, 0, I.stream>>>(P, B, 0, 0);
+    I.launch_br0(0, 0);
     bcoarse_kernel<<<cgrid, 256, 0, I.stream>>>(P, B, B.d, B.alpha, 0, 0);
-    bpnorm_kernel<<<nd, TPB, 0, I.stream>>>(P, B);
+    with_kwidth(P.KS, [&](auto kc) { bpnorm_kernel<decltype(kc)::value><<<I.blk.flat_grid, 256, 0, I.stream>>>(P, B); });
     btol_kernel<<<1, 32, 0, I.stream>>>(P, B);
     CUDA_CHECK(cudaGetLastError());
     const int chunk = std::max(1, I.opt.chunk);
