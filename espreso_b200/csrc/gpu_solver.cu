@@ -2227,7 +2227,11 @@ struct GpuSolver::Impl {
     int el_nd = 0, el_n = 0;
     double *e_dev = nullptr;
     int rho_cap = 0;
-    cudaEvent_t ev0 = nullptr, ev1 = nullptr;
+    void solve_begin(SolveStats &stats);
+    void solve_end(SolveStats &stats);
+    cudaEvent_t ev0 = nullptr, ev1 = nullptr, ev_state = nullptr;
+    DevState *st_host = nullptr;      // pinned: the state after the last solve, in front of h_pinned
+    bool solve_looped = false;
 
     template <typename T>
     T *alloc(size_t n) {
@@ -2254,7 +2258,8 @@ struct GpuSolver::Impl {
     ~Impl() {
         if (blk.graph) cudaGraphExecDestroy(blk.graph);
         if (graph_loop) cudaGraphExecDestroy(graph_loop);
-        if (h_pinned) cudaFreeHost(h_pinned);
+        if (st_host) cudaFreeHost(st_host);   // and h_pinned behind it
+        if (ev_state) cudaEventDestroy(ev_state);
         for (cudaEvent_t e : stage_ev) cudaEventDestroy(e);
         if (graph) cudaGraphExecDestroy(graph);
         for (void *p : allocs) cudaFree(p);
@@ -3220,6 +3225,7 @@ void GpuSolver::upload(const Decomposition &dec, const Prep &prep, const SolveOp
     CUDA_CHECK(cudaStreamCreateWithFlags(&I.stream, cudaStreamNonBlocking));
     CUDA_CHECK(cudaEventCreate(&I.ev0));
     CUDA_CHECK(cudaEventCreate(&I.ev1));
+    CUDA_CHECK(cudaEventCreateWithFlags(&I.ev_state, cudaEventDisableTiming));
     set_smem_limits();
 
     const int nd = dec.ndom;
@@ -3519,10 +3525,14 @@ void GpuSolver::Impl::ensure_pinned(size_t n) {
     n = std::max<size_t>(n, 1);
     if (h_pinned_n >= n) return;
     CUDA_CHECK(cudaStreamSynchronize(stream));   // no copy of the old buffer in flight
-    if (h_pinned) CUDA_CHECK(cudaFreeHost(h_pinned));
+    if (st_host) CUDA_CHECK(cudaFreeHost(st_host));
+    st_host = nullptr;
     h_pinned = nullptr;
     h_pinned_n = 0;
-    CUDA_CHECK(cudaMallocHost(&h_pinned, n * sizeof(double)));
+    constexpr size_t head = 256;   // the state, then the staging buffer on a 256-byte boundary
+    static_assert(sizeof(DevState) <= head, "the solver state fits in front of the staging buffer");
+    CUDA_CHECK(cudaMallocHost(&st_host, head + n * sizeof(double)));
+    h_pinned = reinterpret_cast<double *>(reinterpret_cast<char *>(st_host) + head);
     h_pinned_n = n;
 }
 
@@ -3593,7 +3603,7 @@ void GpuSolver::solve_full(const double *rhs, int rhs_size, double *solution, in
         bvec_kernel<<<(P.NL + 255) / 256, 256, 0, I.stream>>>(P, I.d_rdof, I.d_rsign, I.d_rc, I.d_kf, (double *)P.bL);
         CUDA_CHECK(cudaGetLastError());
     }
-    solve(stats);
+    I.solve_begin(stats);
     // primal: u = K^+ (f - B^T lambda) + R alpha, averaged into the caller's DOFs; Total FETI
     // forms L^-1 (f - B^T lambda) from the kept L^-1 f and a forward pass over the touched blocks
     primal_rhs_kernel<<<std::max(1, std::min(4096, (I.ntot + 255) / 256)), 256, 0, I.stream>>>(
@@ -3604,6 +3614,7 @@ void GpuSolver::solve_full(const double *rhs, int rhs_size, double *solution, in
     CUDA_CHECK(cudaMemsetAsync(I.d_sol, 0, sizeof(double) * std::max(1, I.n_caller), I.stream));
     primal_merge_kernel<<<nd, TPB, 0, I.stream>>>(P, I.d_doff, I.d_rdofs, I.d_Rd, I.d_kf, I.d_gdof, I.d_invm, I.d_sol);
     CUDA_CHECK(cudaGetLastError());
+    I.solve_end(stats);   // the primal kernels run on meanwhile; the caller's array is written after its checks
     const int ncp = std::min(solution_size, I.n_caller);
     I.d2h_columns(solution, 0, I.d_sol, 0, (size_t)std::max(0, ncp), 1);
     for (int i = std::max(0, ncp); i < solution_size; ++i) solution[i] = 0.0;
@@ -3622,8 +3633,14 @@ void GpuSolver::set_rhs(const std::vector<double> &b, const std::vector<double> 
 }
 
 void GpuSolver::solve(SolveStats &stats) {
-    Impl &I = *impl;
-    DevProblem &P = I.P;
+    impl->solve_begin(stats);
+    impl->solve_end(stats);
+}
+
+// The dual PCG on the stream; its final state goes to st_host once ev1 has passed, so that the caller can
+// enqueue what follows before it waits.
+void GpuSolver::Impl::solve_begin(SolveStats &stats) {
+    Impl &I = *this;
     FETI_CHECK(I.opt.max_iterations + 64 <= I.rho_cap, "FETI4I: max_iterations grew after instance creation");
     const bool mixed = I.opt.schur_precision != SCHUR_FP64;
     DevState h{};
@@ -3658,16 +3675,7 @@ void GpuSolver::solve(SolveStats &stats) {
     const bool loop = I.opt.use_graph && I.capture_loop();
     if (I.opt.use_graph && !loop) I.capture_chunk(chunk);
     DevState hs{};
-    if (loop) {
-        CUDA_CHECK(cudaGraphLaunch(I.graph_loop, I.stream));
-        CUDA_CHECK(cudaMemcpyAsync(&hs, I.st, sizeof(hs), cudaMemcpyDeviceToHost, I.stream));
-        CUDA_CHECK(cudaStreamSynchronize(I.stream));
-        const int its = std::max(1, hs.conv_iter >= 0 ? hs.conv_iter + 1 : std::min(hs.iter_base, I.opt.max_iterations));
-        if (loop_kind() == LOOP_SINGLE)
-            launches += its * (I.kernels_per_iteration() + 1) - (mixed ? 2 * (its - hs.replacements) : 0);
-        else
-            launches += (its + LOOP_STEP - 1) / LOOP_STEP * (LOOP_STEP * I.kernels_per_iteration() + 1);
-    }
+    if (loop) CUDA_CHECK(cudaGraphLaunch(I.graph_loop, I.stream));   // no host check: solve_end waits once
     for (int done = 0; !loop && done < I.opt.max_iterations; done += chunk) {
         if (I.opt.use_graph) {
             CUDA_CHECK(cudaGraphLaunch(I.graph, I.stream));
@@ -3684,9 +3692,27 @@ void GpuSolver::solve(SolveStats &stats) {
     coarse_kernel<<<cgrid, 256, 0, I.stream>>>(P, P.d, P.alpha, 0, 0);
     launches += 1;
     CUDA_CHECK(cudaEventRecord(I.ev1, I.stream));
-    CUDA_CHECK(cudaMemcpyAsync(&hs, I.st, sizeof(hs), cudaMemcpyDeviceToHost, I.stream));
-    CUDA_CHECK(cudaStreamSynchronize(I.stream));
+    I.ensure_pinned(1);
+    CUDA_CHECK(cudaMemcpyAsync(I.st_host, I.st, sizeof(DevState), cudaMemcpyDeviceToHost, I.stream));
+    CUDA_CHECK(cudaEventRecord(I.ev_state, I.stream));
+    stats.kernel_launches = launches;
+    I.solve_looped = loop;
+}
+
+void GpuSolver::Impl::solve_end(SolveStats &stats) {
+    Impl &I = *this;
+    CUDA_CHECK(cudaEventSynchronize(I.ev_state));
+    const DevState hs = *I.st_host;
+    const bool mixed = I.opt.schur_precision != SCHUR_FP64;
+    int launches = stats.kernel_launches;
     FETI_CHECK(hs.error == 0, "FETI4I: a device pipeline wait timed out (solve aborted)");
+    if (I.solve_looped) {
+        const int its = std::max(1, hs.conv_iter >= 0 ? hs.conv_iter + 1 : std::min(hs.iter_base, I.opt.max_iterations));
+        if (loop_kind() == LOOP_SINGLE)
+            launches += its * (I.kernels_per_iteration() + 1) - (mixed ? 2 * (its - hs.replacements) : 0);
+        else
+            launches += (its + LOOP_STEP - 1) / LOOP_STEP * (LOOP_STEP * I.kernels_per_iteration() + 1);
+    }
     float ms = 0.f;
     CUDA_CHECK(cudaEventElapsedTime(&ms, I.ev0, I.ev1));
     stats.t_solve_ms = ms;

@@ -1,0 +1,83 @@
+"""Paths of the PCG kernels that the other problems do not reach: a kernel width other than 1 and 6 (two
+uncoupled heat fields: 2 kernel vectors per subdomain), and the default loop graph against the chunked
+graphs."""
+import json
+import os
+import subprocess
+import sys
+
+import numpy as np
+import pytest
+
+from espreso_b200 import feti4i as F
+from espreso_b200 import problems
+from tests.helpers import direct_u
+
+pytestmark = pytest.mark.gpu
+
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+
+
+def two_fields(domains, elements):
+    P = problems.heat_cube(domains=domains, elements=elements, seed=3)
+    Ke = np.zeros((P.Ke.shape[0], 16, 16))
+    fe = np.zeros((P.fe.shape[0], 16))
+    for c in range(2):
+        Ke[:, c::2, c::2] = (1.0 + c) * P.Ke
+        fe[:, c::2] = (1.0 - 3.0 * c) * P.fe
+    fixed = P.dirichlet[0]
+    return problems.Problem("two_fields", 2, P.coords, P.elem_nodes, P.elem_domain, Ke, fe, {0: fixed, 1: fixed}, P.grid)
+
+
+# 8 subdomains: one-CTA kernels and the small coarse problem; 48: clusters, a coarse problem of 96, and more
+# than 8,192 touched DOFs
+@pytest.mark.parametrize("domains,elements", [((2, 2, 2), (3, 3, 3)), ((4, 4, 3), (5, 5, 5))])
+@pytest.mark.parametrize("prec", [F.PREC_NONE, F.PREC_LUMPED, F.PREC_WEIGHT, F.PREC_DIRICHLET])
+def test_kernel_width_two(domains, elements, prec):
+    P = two_fields(domains, elements)
+    inst = problems.make_instance(P, iopts={F.PRECONDITIONER: prec, F.VERBOSE_LEVEL: 0, F.MAX_ITERATIONS: 3000},
+                                  ropts={F.PRECISION: 1e-11})
+    try:
+        ref = direct_u(P)
+        u = inst.solve().reshape(-1, 2)
+        # both solve to 1e-11 of the dual residual; the direct solve is good to about 1e-12
+        assert np.linalg.norm(u - ref) <= 1e-8 * np.linalg.norm(ref)
+        f = P.rhs()
+        U = inst.solve_multi(np.stack([f, -2.0 * f, 0.5 * f]))
+        for j, s in enumerate((1.0, -2.0, 0.5)):
+            assert np.linalg.norm(U[j].reshape(-1, 2) - s * ref) <= 1e-8 * np.linalg.norm(ref)
+    finally:
+        inst.destroy()
+
+
+SCRIPT = r"""
+import json, sys
+sys.path.insert(0, sys.argv[1])
+from espreso_b200 import feti4i as F, problems
+P = problems.elasticity_cube(domains=(3, 2, 2), elements=(3, 3, 3))
+out = {}
+for schur, max_it in ((F.FP64, 2000), (F.FP32, 2000), (F.FP64, 6)):
+    inst = problems.make_instance(P, iopts={F.PRECONDITIONER: F.PREC_LUMPED, F.VERBOSE_LEVEL: 0, F.MAX_ITERATIONS: max_it},
+                                  ropts={F.PRECISION: 1e-10}, ext={F.EXT_SCHUR_PRECISION: schur})
+    u = inst.solve()
+    st = inst.stats()
+    out["%d %d" % (schur, max_it)] = dict(u=u.tolist(), it=st["iterations"], conv=st["converged"])
+    inst.destroy()
+print(json.dumps(out))
+"""
+
+
+def test_default_loop_matches_chunked_graphs():
+    runs = []
+    for env in ({}, {"FETI4I_LOOP_GRAPH": "0"}):
+        clean = {k: v for k, v in os.environ.items() if k != "FETI4I_LOOP_GRAPH"}
+        r = subprocess.run([sys.executable, "-c", SCRIPT, ROOT], capture_output=True, text=True, env=dict(clean, **env),
+                           timeout=600)
+        assert r.returncode == 0, r.stderr
+        runs.append(json.loads(r.stdout.strip().splitlines()[-1]))
+    a, b = runs
+    for key in a:
+        ua, ub = np.array(a[key]["u"]), np.array(b[key]["u"])
+        assert a[key]["it"] == b[key]["it"] and a[key]["conv"] == b[key]["conv"]
+        assert np.linalg.norm(ua - ub) <= 1e-10 * np.linalg.norm(ub)
+    assert a["0 6"]["it"] == 6 and a["0 6"]["conv"] == 0.0   # stopped by max_iterations inside a pass
