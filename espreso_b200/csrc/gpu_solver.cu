@@ -944,17 +944,21 @@ __global__ void coarse_kernel(DevProblem P, const double *in, double *out, int s
     int lane = threadIdx.x & 31;
     if (row >= P.nK) return;
     const double *col = P.GGtinv + (size_t)row * P.nP;
-    // four independent partial sums: the loads of four steps are in flight together
-    double s0 = 0.0, s1 = 0.0, s2 = 0.0, s3 = 0.0;
-    int b = lane;
-    for (; b + 96 < P.nP; b += 128) {
-        s0 += __ldg(col + b) * __ldg(in + b);
-        s1 += __ldg(col + b + 32) * __ldg(in + b + 32);
-        s2 += __ldg(col + b + 64) * __ldg(in + b + 64);
-        s3 += __ldg(col + b + 96) * __ldg(in + b + 96);
+    // sixteen steps in flight together: up to 512 columns take one round trip to L2 (four: 1.65 / 1.575 ms
+    // per solve of 27 subdomains with the Dirichlet preconditioner, 4.97 / 4.88 ms of 64 of 8^3 elements)
+    double s = 0.0;
+    for (int b0 = lane; b0 < P.nP; b0 += 512) {
+        double m[16], v[16];
+#pragma unroll
+        for (int k = 0; k < 16; ++k) {
+            const int b = b0 + 32 * k;
+            m[k] = b < P.nP ? __ldg(col + b) : 0.0;
+            v[k] = b < P.nP ? __ldg(in + b) : 0.0;
+        }
+#pragma unroll
+        for (int k = 0; k < 16; ++k) s += m[k] * v[k];
     }
-    for (; b < P.nP; b += 32) s0 += __ldg(col + b) * __ldg(in + b);
-    double s = warp_sum((s0 + s1) + (s2 + s3));
+    s = warp_sum(s);
     if (lane == 0) out[row] = s;
 }
 
