@@ -4010,6 +4010,93 @@ __device__ __forceinline__ void noalloc_tiles(const uint4 *tiles, int T, int k0,
 __device__ __forceinline__ bool noalloc_valid(int n, int max_order) { return n >= 0 && n <= max_order; }
 __device__ __forceinline__ double noalloc_nan() { return __longlong_as_double(0x7ff8000000000000LL); }
 
+__device__ __forceinline__ double ld_cluster(const double *p, unsigned rank) {
+    unsigned a;
+    double v;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"((unsigned)__cvta_generic_to_shared(p)), "r"(rank));
+    asm volatile("ld.shared::cluster.f64 %0, [%1];" : "=d"(v) : "r"(a) : "memory");
+    return v;
+}
+
+// Whole matrices from a queue, one CTA (CL false) or one cluster of CTAs per matrix: the CTAs of a cluster take
+// runs of its tiles, each into its own y, and sum their y's through distributed shared memory.  For calls
+// whose matrices are short work for a cluster (noalloc_cluster): items cost a set-up kernel first.
+// Latency-bound: a warp has one 8 KB tile in flight, and the steps of a matrix (x, tiles, sums) follow one
+// another.  A CTA per matrix in all cases -> this kernel: 18.6 -> 10.6 us (one matrix of order 400),
+// 34.9 -> 14.5 us (16 of 400-700), 20.7 -> 14.4 us (60 of 200-400), 18.5 -> 16.8 us (300 of 150-250),
+// 78.8 -> 75.9 us (900 of 300-330, 6.4 TB/s).
+template <bool CL>
+__global__ void __launch_bounds__(256, 2)
+tile_symv_noalloc_matrix_kernel(const double *tiles, const long long *tile0, const int *order, const int *voff, int nmat,
+                                int max_order, const double *x, double *y, double *dot_out, NoAllocScratch *scr) {
+    pdl_enter();
+    extern __shared__ __align__(16) double nsm[];
+    __shared__ double red[32];
+    __shared__ double s_next;      // the next matrix (a whole number: it is sent to the cluster's other CTAs)
+    __shared__ int s_last;
+    const int C = CL ? (int)cluster_size_x() : 1, rank = CL ? (int)cluster_rank_x() : 0, ncl = gridDim.x / C;
+    const uint4 *tl = reinterpret_cast<const uint4 *>(tiles);
+    auto barrier = [&] {
+        if (CL) {
+            cluster_arrive();
+            cluster_wait();
+        } else {
+            __syncthreads();
+        }
+    };
+    double dot = 0.0;
+    for (int m = blockIdx.x / C; m < nmat;) {
+        const int n = order[m], o = voff[m];
+        const bool valid = noalloc_valid(n, max_order);
+        const int T = valid ? (n + TILE - 1) / TILE : 0, nt = T * (T + 1) / 2;
+        double *xs = nsm, *ys = nsm + TILE * T;
+        for (int i = threadIdx.x; i < TILE * T; i += blockDim.x) {
+            xs[i] = i < n ? x[o + i] : 0.0;
+            ys[i] = 0.0;
+        }
+        __syncthreads();
+        noalloc_tiles(tl + (size_t)tile0[m] * (TILE * 16), T, nt * rank / C, nt * (rank + 1) / C, xs, ys);
+        barrier();
+        // taken under the sums: any earlier, and a CTA with a large matrix takes work that others would reach first
+        int next = nmat;
+        if (rank == 0 && threadIdx.x == 0 && nmat > ncl) next = ncl + atomicAdd(&scr->queue, 1);
+        if (valid) {
+            for (int i = rank * blockDim.x + threadIdx.x; i < n; i += C * blockDim.x) {
+                double v = CL ? 0.0 : ys[i];
+                if (CL)
+                    for (int r = 0; r < C; ++r) v += ld_cluster(ys + i, (unsigned)r);
+                y[o + i] = v;
+                dot += xs[i] * v;
+            }
+        } else if (rank == 0) {
+            for (int i = threadIdx.x; i < n; i += blockDim.x) y[o + i] = noalloc_nan();
+            dot = noalloc_nan();
+        }
+        if (rank == 0 && threadIdx.x == 0) {
+            if (CL)
+                for (int r = 0; r < C; ++r) st_cluster(&s_next, (unsigned)r, (double)next);
+            else
+                s_next = (double)next;
+        }
+        barrier();                 // ys is read by the cluster until here, s_next is set
+        m = (int)s_next;
+    }
+    dot = block_sum(dot, red);
+    if (threadIdx.x == 0) {
+        scr->dots[blockIdx.x] = dot;
+        __threadfence();
+        s_last = (atomicAdd(&scr->done, 1) == (int)gridDim.x - 1);
+    }
+    __syncthreads();
+    if (s_last) {
+        __threadfence();
+        double t = 0.0;
+        for (int i = threadIdx.x; i < (int)gridDim.x; i += blockDim.x) t += __ldcg(&scr->dots[i]);
+        t = block_sum(t, red);
+        if (threadIdx.x == 0 && dot_out) *dot_out = t;
+    }
+}
+
 // Before the items: y cleared (items of a split matrix add into it), the tiles per item from the number
 // of tiles in all (four items or more per CTA slot, 8 to 48 tiles), the first item of every matrix.  A
 // product in place (y = x) takes whole matrices as items and clears nothing.
@@ -4065,8 +4152,9 @@ __global__ void __launch_bounds__(256) noalloc_setup_kernel(const int *order, co
 
 // Items (runs of tiles of one matrix) from a queue.  With whole matrices as the unit the call waited for
 // the CTA that drew a large one last: 512 matrices of order 333 to 1111 took 250 us a call
-// (4.9 TB/s), 210 us (5.9 TB/s) so; a cluster of CTAs per matrix, which spares the split sums in y, took 242 us: its barriers cost
-// what the balance gave.
+// (4.9 TB/s), 202 us (6.1 TB/s) so; a cluster of CTAs per matrix, which spares the split sums in y, took 242 us: its
+// barriers cost what the balance gave.  The block-wide search and the next item's number taken an item ahead
+// took it from 206 to 202 us against a binary search in every thread.
 __global__ void __launch_bounds__(256, 2)
 tile_symv_noalloc_kernel(const double *tiles, const long long *tile0, const int *order, const int *voff, int nmat,
                          int max_order, const double *x, double *y, double *dot_out, NoAllocScratch *scr) {
@@ -4076,18 +4164,23 @@ tile_symv_noalloc_kernel(const double *tiles, const long long *tile0, const int 
     const uint4 *tl = reinterpret_cast<const uint4 *>(tiles);
     const int nitems = scr->nitems, per = scr->per_item;
     double dot = 0.0;
+    int m = 0;
+    if (threadIdx.x == 0) s_item = atomicAdd(&scr->queue, 1);
+    __syncthreads();
     for (;;) {
-        if (threadIdx.x == 0) s_item = atomicAdd(&scr->queue, 1);
-        __syncthreads();
         const int item = s_item;
         if (item >= nitems) break;
-        int lo = 0, hi = nmat - 1;                     // the matrix whose first item is the last one <= item
-        while (lo < hi) {
-            const int mid = (lo + hi + 1) >> 1;
-            if (scr->first[mid] <= item) lo = mid;
-            else hi = mid - 1;
+        int next = 0;                                  // the next item's number, on its way during this one
+        if (threadIdx.x == 0) next = atomicAdd(&scr->queue, 1);
+        // the matrix whose first item is the last one <= item: a CTA's items ascend, so it lies at or after the
+        // last one, and the CTA looks at 256 matrices at a time
+        for (;;) {
+            const int q = m + (int)threadIdx.x;
+            const int c = __syncthreads_count(q < nmat && scr->first[q] <= item);
+            m += c - 1;
+            if (c < (int)blockDim.x) break;
         }
-        const int m = lo, n = order[m], o = voff[m];
+        const int n = order[m], o = voff[m];
         if (!noalloc_valid(n, max_order)) {
             dot = noalloc_nan();
         } else {
@@ -4109,6 +4202,7 @@ tile_symv_noalloc_kernel(const double *tiles, const long long *tile0, const int 
                 dot += xs[i] * v;
             }
         }
+        if (threadIdx.x == 0) s_item = next;           // every thread has read s_item before the count above
         __syncthreads();
     }
     dot = block_sum(dot, red);
@@ -4183,6 +4277,16 @@ NoAllocScratch *g_noalloc_ptr[256];
 int g_noalloc_nsm[256];
 bool g_noalloc_ready[256];
 
+// CTAs per matrix of the whole-matrix form, 0 for the item form: more CTAs as long as they all run at once and
+// every warp has two tiles.  Items when that leaves a warp more than 8 tiles (some 10 us) of the largest matrix,
+// 14 in one CTA per matrix: whole matrices against items took 41.1 against 45.4 us at 300 matrices of order
+// 330-380, 133 against 141 us at 2,000 of 200-384, 53.7 against 53.5 us at 300 of 384-448 (105 tiles).
+int noalloc_cluster(int nmatrices, int max_tiles, int slots) {
+    int c = 1;
+    while (c < 8 && 2LL * c * nmatrices <= slots && max_tiles >= 16 * c) c *= 2;
+    return max_tiles <= (c == 1 ? 112 : 64 * c) ? c : 0;
+}
+
 }  // namespace
 
 int tiled_symv_noalloc(const double *tiles, const long long *tile_offset, const int *order, const int *vector_offset,
@@ -4212,6 +4316,10 @@ int tiled_symv_noalloc(const double *tiles, const long long *tile_offset, const 
                 cudaFuncSetAttribute(tile_symv_noalloc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
             CUDA_CHECK(cudaFuncSetAttribute(tile_symv_noalloc_small_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                             smem));
+            CUDA_CHECK(cudaFuncSetAttribute(tile_symv_noalloc_matrix_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                            smem));
+            CUDA_CHECK(cudaFuncSetAttribute(tile_symv_noalloc_matrix_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                            smem));
             CUDA_CHECK(cudaDeviceGetAttribute(&g_noalloc_nsm[dev], cudaDevAttrMultiProcessorCount, dev));
             g_noalloc_ptr[dev] = p;
             g_noalloc_ready[dev] = true;
@@ -4227,6 +4335,18 @@ int tiled_symv_noalloc(const double *tiles, const long long *tile_offset, const 
         return 0;
     }
     const int slots = std::min(NOALLOC_MAX_CTAS, 2 * nsm);
+    if (const int c = noalloc_cluster(nmatrices, max_tiles, slots)) {
+        CUDA_CHECK(cudaMemsetAsync(scr, 0, 2 * sizeof(int), s));   // queue and done
+        if (c == 1) {
+            tile_symv_noalloc_matrix_kernel<false><<<std::min(nmatrices, slots), 256, smem, s>>>(
+                tiles, tile_offset, order, vector_offset, nmatrices, max_order, x, y, dot, scr);
+            CUDA_CHECK(cudaGetLastError());
+        } else {
+            launch_cluster(tile_symv_noalloc_matrix_kernel<true>, c, dim3(c * std::min(nmatrices, slots / c)), dim3(256), smem, s,
+                           tiles, tile_offset, order, vector_offset, nmatrices, max_order, x, y, dot, scr);
+        }
+        return 0;
+    }
     // items of 8 tiles or more: no more CTAs than there can be items
     const int grid = (int)std::min<long long>(slots, (long long)nmatrices * ((max_tiles + 7) / 8));
     noalloc_setup_kernel<<<std::min(nmatrices, slots), 256, 0, s>>>(order, vector_offset, nmatrices, max_order, slots, x, y, scr);

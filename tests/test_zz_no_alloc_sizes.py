@@ -1,5 +1,6 @@
-"""FETI4ITiledSymvNoAlloc at the edges of its forms: the one-cluster form and its limit (32 tiles per CTA),
-matrices split into items, ragged and empty orders, many tiny matrices, the product in place."""
+"""FETI4ITiledSymvNoAlloc at the edges of its forms: the one-cluster form and its limit (32 tiles per CTA), a
+cluster per matrix (1 to 8 CTAs, with and without the queue), matrices split into items, ragged and
+empty orders, many tiny matrices, the product in place."""
 import numpy as np
 import pytest
 
@@ -12,7 +13,13 @@ CASES = {
     "one_tile": [32],
     "ragged_9": [33, 0, 1, 31, 32, 64, 65, 17, 100],
     "cluster_limit": [224] * 8,              # 28 tiles each: the largest one-cluster call of eight
-    "above_limit": [225] * 8 + [3],
+    "above_limit": [225] * 8 + [3],          # 36 tiles: four CTAs per matrix
+    "cluster_8": [700, 33, 610],             # 253 tiles: eight
+    "cluster_2": [350] * 100,                # 66 tiles: two
+    "matrix_queue": [300] * 400,             # one CTA each, more matrices than CTAs
+    "matrix_limit": [448, 20] * 160,         # 105 tiles: the largest with one CTA each
+    "above_matrix_limit": [449, 20] * 160,   # 120: items
+    "items_40": [1111] * 5 + [200] * 35,
     "one_large": [1600],
     "mixed": [7, 1000, 32, 640, 0, 333, 96, 1111],
     "many_tiny": [5] * 3000,
